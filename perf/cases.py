@@ -114,6 +114,41 @@ def run(state):
     return pkg.fp8_weight_quant(state["w"])
 
 
+def _groups(x):
+    """[rows, K] bf16 -> (e4m3 values, fp32 scale) per 128-wide group, as [rows, groups, 128] and [rows, groups, 1]."""
+    rows, k = x.shape
+    x = torch.nn.functional.pad(x.float(), (0, -k % 128)).view(rows, -1, 128)
+    s = x.abs().amax(2, keepdim=True)
+    s = s / torch.full_like(s, 448.0)   # (a scalar divisor would become a multiplication by its reciprocal)
+    return torch.where(s > 0, x / s, torch.zeros_like(x)).to(torch.float8_e4m3fn), s
+
+
+def _blocks(w):
+    """[N, K] bf16 -> (e4m3 values, fp32 scale) per 128 x 128 block, as [Nb, 128, Kb, 128] and [Nb, 1, Kb, 1]."""
+    n, k = w.shape
+    w = torch.nn.functional.pad(w.float(), (0, -k % 128, 0, -n % 128)).view(-(-n // 128), 128, -(-k // 128), 128)
+    s = w.abs().amax((1, 3), keepdim=True)
+    s = s / torch.full_like(s, 448.0)
+    return torch.where(s > 0, w / s, torch.zeros_like(w)).to(torch.float8_e4m3fn), s
+
+
+def exact(case, seed):
+    op, m, n, k = case["op"], case["M"], case["N"], case["K"]
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(seed)
+    if op != "weight_quant":
+        qx, sx = _groups(torch.randn(m, k, generator=g, device=dev, dtype=torch.bfloat16))
+        if op == "act_quant":
+            return None, sx.double()[:, :, 0]   # the bytes are compared as such
+    w = torch.randn(n, k, generator=g, device=dev, dtype=torch.bfloat16).mul_(0.02)
+    qw, sw = _groups(w) if op == "rowscale" else _blocks(w)
+    if op == "weight_quant":
+        return None, sw.double()[:, 0, :, 0]
+    a = (qx.double() * sx.double()).view(m, -1)
+    b = (qw.double() * sw.double()).view(-1, a.shape[1])[:n]
+    return a @ b.T
+
+
 def work(case):
     op, m, n, k = case["op"], case["M"], case["N"], case["K"]
     kb, nb = -(-k // 128), -(-n // 128)
