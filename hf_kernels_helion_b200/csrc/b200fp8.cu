@@ -558,16 +558,25 @@ int b200fp8_quant_act(const void* x, void* q, float* s, int64_t M, int64_t K, in
   if (K % 128 == 0 && (M == 1 || (ldx == K && ldq == K && lds == K / 128)) &&
       (reinterpret_cast<uintptr_t>(q) & 15u) == 0 && groups <= (int64_t{1} << 35)) {
     // one unbroken run of 128-element groups: no row / column arithmetic in the kernel
-    const int64_t blocks = (groups + 31) / 32;
-    quant_act_contig_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
+    const unsigned blocks = static_cast<unsigned>((groups + 63) / 64);
+    if ((reinterpret_cast<uintptr_t>(x) & 31u) == 0)
+      quant_act_contig_kernel<true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
+    else
+      quant_act_contig_kernel<false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
     return launch_status();
   }
   const int64_t blocks_needed = (groups * 8 + 255) / 256;
   const int64_t max_blocks = static_cast<int64_t>(dev->sm_count) * 32;
   const int grid = static_cast<int>(blocks_needed < max_blocks ? blocks_needed : max_blocks);
-  quant_act_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
+  // (the last pass of the loop steps at most one grid beyond the padded count)
+  if (groups + 4 + static_cast<int64_t>(grid) * 32 <= 0xFFFFFFFFll)
+    quant_act_kernel<uint32_t><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
+  else
+    quant_act_kernel<int64_t><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
   return launch_status();
 }
 
@@ -585,8 +594,14 @@ int b200fp8_quant_weight(const void* w, void* q, float* s, int64_t N, int64_t K,
   if (st != B200FP8_OK) return st;
   const int64_t blocks = ((N + 127) / 128) * ((K + 127) / 128);
   if (blocks > 0x7FFFFFFF) return B200FP8_ERR_TOO_LARGE;
-  quant_weight_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(w), static_cast<uint8_t*>(q), s, N, K, ldw, ldq, lds);
+  const bool wide = K % 16 == 0 && ldw % 16 == 0 && ldq % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 31u) == 0 &&
+                    (reinterpret_cast<uintptr_t>(q) & 15u) == 0;
+  if (wide)
+    quant_weight_kernel<true><<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(w), static_cast<uint8_t*>(q), s, N, K, ldw, ldq, lds);
+  else
+    quant_weight_kernel<false><<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(w), static_cast<uint8_t*>(q), s, N, K, ldw, ldq, lds);
   return launch_status();
 }
 

@@ -967,10 +967,11 @@ __global__ void __launch_bounds__(256)
 tile_prep_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, uint8_t* __restrict__ Aq, int64_t ldq,
                        int64_t rows_q, float* __restrict__ AsT, int64_t M, int64_t m_pad, int num_kb) {
   asm volatile("griddepcontrol.launch_dependents;");
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-  const int64_t g = t >> 3;
+  const int64_t g = static_cast<int64_t>(blockIdx.x) * 32 + (threadIdx.x >> 3);
   const int sub = threadIdx.x & 7;
-  const int64_t row = g / num_kb;                 // whole warps share a row quadruple: m_pad * num_kb is a multiple of 4
+  // (the 64-bit division costs several times the 32-bit one)
+  const int64_t row = g <= 0x7fffffff ? static_cast<int64_t>(static_cast<uint32_t>(g) / static_cast<uint32_t>(num_kb))
+                                      : g / num_kb;   // whole warps share a row quadruple: m_pad * num_kb is a multiple of 4
   const int kg = static_cast<int>(g - row * num_kb);
   if (row >= m_pad) return;
   uint4 v[2];

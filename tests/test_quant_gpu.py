@@ -198,3 +198,16 @@ def test_quant_feeds_gemm_layout(device):
     assert oracle.max_err_over_rms(out.cpu(), ref) < 1e-4
     y = pkg.fp8_linear(a.to(device).view(4, 16, 512), wq, ws)
     assert y.shape == (4, 16, 256) and y.dtype == torch.bfloat16
+
+
+@pytest.mark.parametrize("rows,K,offset,ld", [(65, 256, 0, 256), (65, 256, 8, 256), (33, 128, 16, 128), (129, 272, 0, 272),
+                                              (129, 264, 0, 264), (130, 256, 16, 272), (130, 256, 8, 264), (1, 8, 8, 8)])
+def test_quantisers_over_alignments(device, rows, K, offset, ld):
+    """Base addresses and pitches that are multiples of 16 bytes but not of 32, and K not a multiple of 16, against
+    ones that are: 256-bit loads are taken only where every piece is aligned, and the bytes are the same."""
+    g = torch.Generator().manual_seed(rows + K + offset)
+    flat = torch.randn(offset + rows * ld, generator=g).to(torch.bfloat16).to(device)
+    x = flat[offset:].view(rows, ld)[:, :K]
+    assert x.data_ptr() % 32 == (offset * 2) % 32
+    _assert_bit_exact(*pkg.fp8_act_quant(x), *oracle.quant_act(x.cpu().contiguous()))
+    _assert_bit_exact(*pkg.fp8_weight_quant(x), *oracle.quant_weight(x.cpu().contiguous()))
