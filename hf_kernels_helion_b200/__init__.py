@@ -9,6 +9,7 @@ Additions that the reference does not have are ``fp8_act_quant``, ``fp8_weight_q
 from __future__ import annotations
 
 import torch
+from torch.compiler import is_compiling
 
 from . import runtime
 from ._ops import ops
@@ -17,6 +18,10 @@ from .op import w8a8_block_fp8_matmul as _m
 from .op import w8a8_block_fp8_matmul_out as _mo
 from .runtime import check_device_status
 
+# The functions below take ordinary eager CUDA calls through one native function (csrc/torch_call.cpp), which
+# answers None for every call that it does not know to be one; those go on through the registered ops and
+# runtime.py, and so does everything under torch.compile. The two ways launch the same kernels; call after call on one
+# stream a 512 x 512 x 2048 product takes 12.8 us this way and 50.4 us the other, a small quantisation 5.2 and 31.9 us.
 _OUT_CODE = {torch.bfloat16: 0, torch.float32: 1}
 
 
@@ -30,6 +35,12 @@ def w8a8_block_fp8_matmul(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs
     The reference's own harness (finegrained-fp8-helion/bench.py:25-28) still calls this function
     in an older form, `w8a8_block_fp8_matmul(A, B, sA, sB, 128)`: an int block size and one B scale
     per ROW of B, sB [N, K // 128].  That form is accepted too and runs the row-scaled kernel."""
+    if not is_compiling():
+        native = runtime.native or runtime.native_for(A)
+        if native is not None:
+            res = native.matmul(A, B, As, Bs, block_size, output_dtype)
+            if res is not None:
+                return res
     if isinstance(block_size, int):
         res = runtime.gemm_rowscale(A, B, As, Bs, block_size,
                                     output_dtype if output_dtype in _OUT_CODE else torch.float32)
@@ -46,11 +57,23 @@ def w8a8_block_fp8_matmul(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs
 def fp8_act_quant(x: torch.Tensor, block_size: int = 128):
     """Per-token-group quantiser: x [M, K] bf16 -> (q [M, K] float8_e4m3fn, s [M, K // 128] fp32)
     with s = group amax / 448 and q = e4m3(x / s).  No counterpart in the reference."""
+    if not is_compiling():
+        native = runtime.native or runtime.native_for(x)
+        if native is not None:
+            res = native.act_quant(x, block_size)
+            if res is not None:
+                return res
     return ops.fp8_act_quant(x, int(block_size))
 
 
 def fp8_weight_quant(w: torch.Tensor, block_size: int = 128):
     """128x128-block quantiser: w [N, K] bf16 -> (q [N, K] float8_e4m3fn, s [N // 128, K // 128] fp32)."""
+    if not is_compiling():
+        native = runtime.native or runtime.native_for(w)
+        if native is not None:
+            res = native.weight_quant(w, block_size)
+            if res is not None:
+                return res
     return runtime.quant_weight(w, int(block_size))
 
 
@@ -62,6 +85,12 @@ def fp8_linear(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor
     layout; measured 2 us faster at M <= 64, N = 28672); larger inputs run the quantiser and the
     matmul as two calls, which is faster there (1148 vs 1242 us at 8192 x 18432 x 7168).
     Same values either way."""
+    if not is_compiling():
+        native = runtime.native or runtime.native_for(x)
+        if native is not None:
+            y = native.linear(x, weight, weight_scale, output_dtype)
+            if y is not None:
+                return y
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     if (x2.shape[0] <= 256 and x2.shape[1] % 128 == 0 and x2.dtype == torch.bfloat16

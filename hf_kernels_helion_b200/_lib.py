@@ -10,6 +10,7 @@ from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libb200fp8.so"
+NATIVE_PATH = LIB_PATH.with_name("_torch_call.so")
 
 OUT_BF16, OUT_FP32 = 0, 1
 VARIANT_AUTO, VARIANT_TILE128, VARIANT_TILE256, VARIANT_STREAMK, VARIANT_TILE256_SK = 0, 1, 2, 3, 4
@@ -73,6 +74,20 @@ def load():
             fn.argtypes = argtypes
         _lib = lib
     return _lib
+
+
+def load_native():
+    """The module built from csrc/torch_call.cpp, bound to the library; raise if either has not been built."""
+    lib = load()
+    try:
+        from . import _torch_call
+    except ImportError as e:
+        raise RuntimeError(f"{NATIVE_PATH} is missing or does not load ({e}): build it with "
+                           "`python -m hf_kernels_helion_b200.build`") from e
+    _torch_call.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
+        "b200fp8_gemm", "b200fp8_gemm_workspace_bytes", "b200fp8_gemm_rowscale", "b200fp8_gemm_rowscale_workspace_bytes",
+        "b200fp8_linear", "b200fp8_linear_workspace_bytes", "b200fp8_quant_act", "b200fp8_quant_weight")))
+    return _torch_call
 
 
 def strerror(status: int) -> str:

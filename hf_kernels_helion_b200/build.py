@@ -1,4 +1,4 @@
-"""Build libb200fp8.so (sm_100a only) next to this file with nvcc.
+"""Build libb200fp8.so (sm_100a only) next to this file with nvcc, and _torch_call.so beside it with g++.
 
     python -m hf_kernels_helion_b200.build [--force] [--verbose]
 
@@ -18,6 +18,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libb200fp8.so"
 SOURCES = [CSRC / "b200fp8.cu"]
+NATIVE_PATH = PKG_DIR / "_torch_call.so"   # host side of the Python calls: links torch, has no kernels
+NATIVE_SOURCES = [CSRC / "torch_call.cpp", PKG_DIR.parent / "include" / "b200fp8.h"]
 HEADERS = sorted(CSRC.glob("*.cuh")) + [PKG_DIR.parent / "include" / "b200fp8.h"]
 
 NVCC_FLAGS = [
@@ -34,25 +36,48 @@ def find_nvcc() -> str:
     return nvcc
 
 
+def _is_stale(target: Path, sources) -> bool:
+    return not target.exists() or any(p.stat().st_mtime > target.stat().st_mtime for p in sources)
+
+
 def is_stale() -> bool:
-    if not LIB_PATH.exists():
-        return True
-    built = LIB_PATH.stat().st_mtime
-    return any(p.stat().st_mtime > built for p in SOURCES + HEADERS)
+    return _is_stale(LIB_PATH, SOURCES + HEADERS) or _is_stale(NATIVE_PATH, NATIVE_SOURCES)
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [find_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += ["-o", str(LIB_PATH), *map(str, SOURCES)]
+def _native_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    root = str(Path(find_nvcc()).resolve().parent.parent)
+    includes = cpp_extension.include_paths() + [sysconfig.get_path("include"), os.path.join(root, "include")]
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in includes:
+        cmd += ["-isystem", d]
+    cmd += [str(NATIVE_SOURCES[0]), "-o", str(NATIVE_PATH)]
+    for d in cpp_extension.library_paths():
+        cmd += ["-L", d]
+    return cmd + ["-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"]
+
+
+def _run(cmd, verbose: bool) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
-        raise RuntimeError(f"nvcc failed with exit code {res.returncode}")
+        raise RuntimeError(f"{Path(cmd[0]).name} failed with exit code {res.returncode}")
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    if force or _is_stale(LIB_PATH, SOURCES + HEADERS):
+        cmd = [find_nvcc(), *NVCC_FLAGS]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        _run(cmd + ["-o", str(LIB_PATH), *map(str, SOURCES)], verbose)
+    if force or _is_stale(NATIVE_PATH, NATIVE_SOURCES):
+        _run(_native_command(), verbose)
     return LIB_PATH
 
 

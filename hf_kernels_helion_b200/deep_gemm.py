@@ -12,6 +12,7 @@ from __future__ import annotations
 import hashlib
 
 import torch
+from torch.compiler import is_compiling
 
 from . import runtime
 
@@ -32,6 +33,13 @@ def _(A, B, As, Bs, block_k):
 
 def gemm_fp8_fp8_bf16_nt(A, B, As, Bs, block_size=128):
     """DeepGEMM-style blockwise fp8 GEMM (NT layout): (A*As) @ (B*Bs)^T -> bf16."""
+    if not is_compiling():
+        native = runtime.native or runtime.native_for(A)
+        # (an int block size is the row-scaled form of the native call)
+        if native is not None and isinstance(block_size, int):
+            res = native.matmul(A, B, As, Bs, block_size, torch.bfloat16)
+            if res is not None:
+                return res
     return getattr(torch.ops, OPS_NAME).gemm_fp8_fp8_bf16_nt(A, B, As, Bs, int(block_size))
 
 

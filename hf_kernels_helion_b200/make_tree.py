@@ -8,13 +8,13 @@ directory, `metadata.json`, and a sub-directory named like the kernel whose `__i
 flat `__init__.py` by path) so that `PYTHONPATH=OUT_DIR/torch-cuda` makes
 `import finegrained_fp8_helion` resolve to this implementation:
 
-    OUT_DIR/torch-cuda/__init__.py _ops.py op.py runtime.py _lib.py tp.py libb200fp8.so metadata.json
+    OUT_DIR/torch-cuda/__init__.py _ops.py op.py runtime.py _lib.py tp.py libb200fp8.so _torch_call.so metadata.json
     OUT_DIR/torch-cuda/finegrained_fp8_helion/__init__.py
     OUT_DIR/benchmarks/benchmark.py        setup / benchmark_* / verify_* for kernels.benchmark
 
 `metadata.json` keeps the reference's name, id and backend and has an empty `python-depends`
 (the reference's is ["helion"], build.toml:9). The tree is binary: it carries the built
-`libb200fp8.so`, not the CUDA sources.
+`libb200fp8.so` and `_torch_call.so`, not the sources.
 """
 from __future__ import annotations
 
@@ -119,6 +119,7 @@ def make_tree(out_dir: Path) -> Path:
     for name in MODULES:
         shutil.copy2(pkg / name, root / name)
     shutil.copy2(lib, root / lib.name)
+    shutil.copy2(_build.NATIVE_PATH, root / _build.NATIVE_PATH.name)
     meta = {
         "name": "finegrained-fp8-helion",
         "id": "_finegrained_fp8_helion_cuda_b0d7177",

@@ -46,7 +46,24 @@ def status_word(device: torch.device) -> torch.Tensor:
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
         _status_words[idx] = w
+        if native is not None:
+            native.set_status(idx, w.data_ptr())
     return w
+
+
+# csrc/torch_call.cpp, bound to the loaded library on the first call with a CUDA tensor
+native = None
+
+
+def native_for(t):
+    """The native call module, or None for what is not a CUDA tensor (the Python path reports that)."""
+    global native
+    if native is None and isinstance(t, torch.Tensor) and t.is_cuda:
+        mod = _lib.load_native()
+        for idx, w in list(_status_words.items()):
+            mod.set_status(idx, w.data_ptr())
+        native = mod
+    return native
 
 
 def check_device_status(device=None) -> None:
