@@ -66,7 +66,7 @@ int device_info(const DeviceInfo** out) {
       opt_in(reinterpret_cast<const void*>(&gemm_tile_kernel<256, 0>), TileCfg<256, false>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_multi_kernel<128>), TileCfg<128, true>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_multi_kernel<256>), TileCfg<256, true>::SMEM_BYTES);
-      opt_in(reinterpret_cast<const void*>(&gemm_tile_rowb_kernel<128>), TileCfg<128, false>::SMEM_BYTES + kRowbTableBytes);
+      opt_in(reinterpret_cast<const void*>(&gemm_tile_rowb_kernel<128>), TileCfg<128, false, 128, 0, true>::SMEM_BYTES);
       regs_ok(reinterpret_cast<const void*>(&gemm_tile_rowb_kernel<128>), TileCfg<128>::THREADS,
               128 * TileCfg<128>::REGS_CONTROL + 256 * TileCfg<128>::REGS_EPILOGUE);
       regs_ok(reinterpret_cast<const void*>(&gemm_tile_kernel<128, 0>), TileCfg<128>::THREADS,
@@ -90,6 +90,13 @@ int device_info(const DeviceInfo** out) {
               128 * TileCfg<256>::REGS_CONTROL + 256 * TileCfg<256>::REGS_EPILOGUE);
       using PairCfg = TileCfg<256, false, 128, 1>;
       using PairMultiCfg = TileCfg<256, true, 128, 1>;
+      using PairRowbCfg = TileCfg<256, true, 128, 2, true>;
+      opt_in(reinterpret_cast<const void*>(&gemm_pair_rowb_kernel<0>), PairRowbCfg::SMEM_BYTES);
+      opt_in(reinterpret_cast<const void*>(&gemm_pair_rowb_kernel<1>), PairRowbCfg::SMEM_BYTES);
+      regs_ok(reinterpret_cast<const void*>(&gemm_pair_rowb_kernel<0>), PairRowbCfg::THREADS,
+              128 * PairRowbCfg::REGS_CONTROL + 256 * PairRowbCfg::REGS_EPILOGUE);
+      regs_ok(reinterpret_cast<const void*>(&gemm_pair_rowb_kernel<1>), PairRowbCfg::THREADS,
+              128 * PairRowbCfg::REGS_CONTROL + 256 * PairRowbCfg::REGS_EPILOGUE);
       opt_in(reinterpret_cast<const void*>(&gemm_pair_kernel<false>), PairCfg::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_pair_kernel<true>), PairCfg::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_pair_multi_kernel<false>), PairMultiCfg::SMEM_BYTES);
@@ -172,7 +179,7 @@ struct TmapKey {
   const void* base;
   int64_t rows, cols, ld;
   uint32_t box_rows;
-  int kind;   // 0: byte matrix, 128-byte boxes, SWIZZLE_128B; 1: fp32 matrix, 128-element boxes, no swizzle
+  int kind;   // 0: byte matrix, 128-byte boxes, SWIZZLE_128B; 1, 2: fp32 matrix, 128- or 256-element boxes, no swizzle
   bool operator==(const TmapKey& o) const {
     return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && kind == o.kind;
   }
@@ -185,7 +192,8 @@ struct TmapCache {
 };
 thread_local TmapCache t_tmap_cache;
 
-// kind 0: byte matrix [rows, cols], ld in bytes; kind 1: fp32 matrix [rows, cols], ld in bytes, box = [box_rows x 128 floats]
+// kind 0: byte matrix [rows, cols], ld in bytes; kind 1 / 2: fp32 matrix [rows, cols], ld in bytes, box = [box_rows x
+// 128 / 256 floats]
 int make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, uint32_t box_rows, int kind) {
   const TmapKey k = {base, rows, cols, ld, box_rows, kind};
   TmapCache& c = t_tmap_cache;
@@ -198,11 +206,11 @@ int make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, in
   if (fn == nullptr) return B200FP8_ERR_DRIVER;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld)};
-  const cuuint32_t box[2] = {128u, box_rows};
+  const cuuint32_t box[2] = {kind == 2 ? 256u : 128u, box_rows};
   const cuuint32_t elem[2] = {1u, 1u};
-  const CUresult r = fn(map, kind == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+  const CUresult r = fn(map, kind >= 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
                         const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        kind == 1 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                        kind >= 1 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return B200FP8_ERR_DRIVER;
   const int slot = c.used < kTmapCacheEntries ? c.used++ : c.next;
@@ -286,6 +294,9 @@ int64_t linear_prefix_bytes(int64_t M, int64_t K) {
   if (M == 0 || K == 0) return 0;
   return tile_ast_bytes(M, K) + align_up((M < 16 ? 16 : M) * align_up(K, 16), 256);
 }
+
+// row-scaled B: the K-block-major copy of the B scales
+int64_t bst_bytes(int64_t N, int64_t K) { return align_up(((K + 127) / 128) * align_up(N, 128) * 4, 256); }
 
 // 128x256 tiles with the last, partly empty wave split along K (B200FP8_VARIANT_TILE256_SK)
 struct TileSkPlan {
@@ -380,6 +391,25 @@ int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   return worth ? B200FP8_VARIANT_TILE256_SK : B200FP8_VARIANT_TILE256;
 }
 
+// Row-scaled B: 128 x 128 tiles, or 256 x 256 tiles on CTA pairs (with the last wave split along K where that can be
+// done), whichever a straight-line fit to measured times says is faster. Per wave and K block a 128 x 128 tile takes
+// 0.56 us and a pair tile, four times the area on two SMs, 0.87; both start with about 8 us of launches and
+// prologue, the fix-up pass of the split tail takes 5. Measured, 128 x 128 / pair / pair with split tail, us:
+// 4096 x 4096 x 8192 268.6 / 241.8 / 221.8, 2048 x 2048 x 4096 46.8 / 36.9 / 36.8, 256 x 4096 x 4096 25.2 / 35.1 / 20.5,
+// 512 x 2048 x 2048 16.7 / 22.0 / 17.6, 8192 x 4096 x 7168 469.8 / 386.4 / 395.5.
+int pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
+  if (pairs < 1 || M <= 128) return B200FP8_VARIANT_TILE128;
+  const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
+  const double kb = static_cast<double>((K + 127) / 128);
+  const double t128 = 0.56 * kb * static_cast<double>((tiles + sm_count - 1) / sm_count);
+  const TileSkPlan p = pair_sk_plan(M, N, K, pairs);
+  const double full = 0.87 * kb * static_cast<double>(p.full / pairs);
+  const double t_pair = full + (p.tail > 0 ? 0.87 * kb : 0.0);
+  const double t_sk = p.split >= 2 ? full + 0.87 * p.kb_per + 5.0 : t_pair;
+  if (t128 <= t_pair && t128 <= t_sk) return B200FP8_VARIANT_TILE128;
+  return t_sk < t_pair ? B200FP8_VARIANT_PAIR256_SPLIT_SK : B200FP8_VARIANT_PAIR256_SPLIT;
+}
+
 template <int BN>
 int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda, int64_t ldb, int sm_count,
                 cudaStream_t stream, int64_t sk_grid = 0) {
@@ -426,7 +456,7 @@ int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda,
     st = make_tmap(&tbst, args.BsT, kblocks, args.n_pad, args.n_pad * 4,
                    static_cast<uint32_t>(kblocks < kRowbTableKb ? kblocks : kRowbTableKb), 1);
     if (st != B200FP8_OK) return st;
-    cfg.dynamicSmemBytes = TileCfg<128, false>::SMEM_BYTES + kRowbTableBytes;
+    cfg.dynamicSmemBytes = TileCfg<128, false, 128, 0, true>::SMEM_BYTES;
     err = cudaLaunchKernelEx(&cfg, gemm_tile_rowb_kernel<128>, ta, tb, tbst, args);
   } else if (args.mc_store) {
     cfg.dynamicSmemBytes = TileCfg<BN, true>::SMEM_BYTES;
@@ -493,7 +523,14 @@ int launch_pair(const void* A, const void* B, const GemmArgs& args, int64_t lda,
       if (st != B200FP8_OK) return st;
     }
     cfg.dynamicSmemBytes = TileCfg<256, true, 128, 1>::SMEM_BYTES;
-    if (args.sk_split >= 2) err = cudaLaunchKernelEx(&cfg, gemm_pair_multi_sk_kernel, ta, tb, args, dm);   // (SPLIT form only)
+    if (args.BsT != nullptr) {
+      CUtensorMap tbst;
+      st = make_tmap(&tbst, args.BsT, (args.K + 127) / 128, args.n_pad, args.n_pad * 4, kRowbChunkKb, 2);
+      if (st != B200FP8_OK) return st;
+      cfg.dynamicSmemBytes = TileCfg<256, true, 128, 2, true>::SMEM_BYTES;
+      err = args.sk_split >= 2 ? cudaLaunchKernelEx(&cfg, gemm_pair_rowb_kernel<1>, ta, tb, tbst, args, dm)
+                               : cudaLaunchKernelEx(&cfg, gemm_pair_rowb_kernel<0>, ta, tb, tbst, args, dm);
+    } else if (args.sk_split >= 2) err = cudaLaunchKernelEx(&cfg, gemm_pair_multi_sk_kernel, ta, tb, args, dm);   // (SPLIT form only)
     else err = cudaLaunchKernelEx(&cfg, gemm_pair_multi_kernel<SPLIT>, ta, tb, args, dm);
   } else {
     cfg.dynamicSmemBytes = TileCfg<256, false, 128, 1>::SMEM_BYTES;
@@ -672,8 +709,6 @@ struct FusedQuant {
   bool rowb = false;
 };
 
-int64_t bst_bytes(int64_t N, int64_t K) { return align_up(((K + 127) / 128) * align_up(N, 128) * 4, 256); }
-
 static int gemm_impl(bool mc, const void* A, const void* B, const float* As, const float* Bs, int n_dst, void* const* dst,
                      const int64_t* dst_ld, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ld_as,
                      int64_t ld_bs, int out_dtype, int variant, void* workspace, size_t workspace_bytes,
@@ -737,7 +772,14 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
   const bool auto_variant = variant == B200FP8_VARIANT_AUTO;
   // (the pair form only pays with the staged output: a destination that cannot take 16-byte rows gets the single-CTA choice)
   if (auto_variant) variant = pick_variant(M, N, K, dev->sm_count, (staged && !mc && !fq.rowb) ? dev->pair_clusters : 0);
-  if (fq.rowb) variant = B200FP8_VARIANT_TILE128;   // the row-scaled promotion exists for the 128-wide tile only
+  if (fq.rowb) {
+    variant = pick_rowb(M, N, K, dev->sm_count, staged ? dev->pair_clusters : 0);
+    // (a workspace without room for the partial tiles: the same tiles without the split tail)
+    if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK &&
+        static_cast<int64_t>(workspace_bytes) < tile_workspace_bytes(M, K) + bst_bytes(N, K) +
+                                                    pair_sk_plan(M, N, K, dev->pair_clusters).partial_bytes)
+      variant = B200FP8_VARIANT_PAIR256_SPLIT;
+  }
   const bool multi = n_dst > 1 || mc;
   if (fq.rowb && (multi || fused_q)) return B200FP8_ERR_VARIANT;
   // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room
@@ -751,7 +793,7 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     variant = B200FP8_VARIANT_PAIR256_SPLIT;   // (2 GPUs, 8192 x 18432 x 7168: 0.596 vs 0.608 ms for the unsplit form)
   const bool pair = variant == B200FP8_VARIANT_PAIR256 || variant == B200FP8_VARIANT_PAIR256_SPLIT ||
                     variant == B200FP8_VARIANT_PAIR256_SPLIT_SK;
-  if (pair && (mc || fq.rowb)) return B200FP8_ERR_VARIANT;
+  if (pair && mc) return B200FP8_ERR_VARIANT;
   if (multi && !pair && variant != B200FP8_VARIANT_TILE128 && variant != B200FP8_VARIANT_TILE256)
     return B200FP8_ERR_VARIANT;
 
@@ -806,7 +848,7 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     args.n_pad = align_up(N, 128);
     if (fq.rowb) {
       // second transposition: the row scales of B, K-block-major (same kernel, B in the role of A)
-      float* bst = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix);
+      float* bst = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix + (sk ? skp.partial_bytes : 0));
       const dim3 grid(static_cast<unsigned>(args.n_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
       tile_prep_kernel<<<grid, 256, 0, stream>>>(Bs, bst, N, args.n_pad, static_cast<int>(kblocks), ld_bs, nullptr,
                                                  nullptr, K, 0, 0);
@@ -923,7 +965,9 @@ int b200fp8_gemm_rowscale(const void* A, const void* B, const float* As, const f
 int64_t b200fp8_gemm_rowscale_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M < 0 || N < 0 || K < 0) return -static_cast<int64_t>(B200FP8_ERR_SHAPE);
   if (M == 0 || N == 0 || K == 0) return 0;
-  return tile_workspace_bytes(M, K) + bst_bytes(N, K);
+  const int pairs = b200fp8_gemm_pair_clusters();
+  const bool sk = pick_rowb(M, N, K, sm_count_or_default(), pairs) == B200FP8_VARIANT_PAIR256_SPLIT_SK;
+  return tile_workspace_bytes(M, K) + bst_bytes(N, K) + (sk ? pair_sk_plan(M, N, K, pairs).partial_bytes : 0);
 }
 
 int b200fp8_linear(const void* x_bf16, const void* B, const float* Bs, void* C, int64_t M, int64_t N, int64_t K,

@@ -80,6 +80,14 @@ struct GemmArgs {
   uint32_t* status_word;
 };
 
+// Row-scaled kernels, per-column B scales in shared memory. 128-wide tile: all K blocks of a tile at once, up to
+// kRowbTableKb (128 floats each). CTA pairs: a ring of kRowbChunks chunks of kRowbChunkKb K blocks (256 floats
+// each), 8 KiB a chunk; three of them let the producer run its whole operand ring ahead of the promotion
+// without waiting for a chunk, whatever K is.
+constexpr int kRowbTableKb = 64;
+constexpr int kRowbChunkKb = 8;
+constexpr int kRowbChunks = 3;
+
 // A_ROWS_: rows of A that the TMA actually brings in per K block (128; 16 or 64 for decode shapes
 // with M <= 16 / M <= 64). The MMA always reads 128 rows from the A slot; with a short slot
 // (2 or 8 KiB) the remaining rows alias the B tile that follows it in the same stage - garbage
@@ -92,7 +100,7 @@ struct GemmArgs {
 // block as two 128-column halves with a TMEM-full / TMEM-empty barrier pair each: the promotion of
 // columns 0..127 starts when the first half of the MMAs has retired and its TMEM columns are handed
 // back a half block earlier, which shortens the accumulator round trip that bounds the kernel.
-template <int BN_, bool MULTI_ = false, int A_ROWS_ = 128, int PAIR_ = 0>
+template <int BN_, bool MULTI_ = false, int A_ROWS_ = 128, int PAIR_ = 0, bool ROWB_ = false>
 struct TileCfg {
   static constexpr int BM = 128;                          // rows per CTA
   static constexpr int PAIR = PAIR_;
@@ -123,8 +131,9 @@ struct TileCfg {
   // warpgroups take them. setmaxnreg.inc BLOCKS until the registers exist, so the sum must
   // not exceed what the launch allocated.
   static constexpr int REGS_LAUNCH = 168;
-  static constexpr int REGS_CONTROL = 56;
-  static constexpr int REGS_EPILOGUE = 224;
+  // (The row-scaled pair kernel takes all that the launch has: 428 bytes of spills with 224, 16-56 with 232.)
+  static constexpr int REGS_CONTROL = (ROWB_ && PAIR_) ? 40 : 56;
+  static constexpr int REGS_EPILOGUE = (ROWB_ && PAIR_) ? 232 : 224;
   static_assert(128 * REGS_CONTROL + 32 * EPI_WARPS * REGS_EPILOGUE <= REGS_LAUNCH * THREADS,
                 "setmaxnreg.inc would wait for registers that never become free");
   static constexpr int A_BYTES = A_ROWS_ * BK;
@@ -143,7 +152,8 @@ struct TileCfg {
   // loop and the warp idles while the link drains. Two boxes (pair kernels, whose smaller pipeline
   // stages leave the room) let a whole bf16 tile queue up behind the K loop of the next one. Measured,
   // 8192 x 18432 x 7168 N-sharded: 2 GPUs 590 vs 611 us for the single-CTA form with one box; 4 GPUs 538 vs 540.
-  static constexpr int OUT_BUFS = (MULTI_ && PAIR_) ? 2 : 1;
+  // (The row-scaled pair kernel has one box: its scale chunks take the room of the second.)
+  static constexpr int OUT_BUFS = (MULTI_ && PAIR_ && !ROWB_) ? 2 : 1;
   static constexpr int OUT_BOX_BYTES = 32 * 128;
   static constexpr int OUT_STAGE_BYTES_PER_WARP = OUT_BOX_BYTES * OUT_BUFS;
   // (MULTI_ instantiations stage their output; the host takes them for several destinations and,
@@ -153,17 +163,17 @@ struct TileCfg {
   // instantiations store straight from registers.)
   static constexpr bool MULTI = MULTI_;
   static constexpr int OUT_STAGE_BYTES = MULTI_ ? EPI_WARPS * OUT_STAGE_BYTES_PER_WARP : 0;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_STAGE_BYTES + BAR_BYTES + 1024;  // +1024: alignment slack
+  // row-scaled kernels: the B scales in shared memory (see kRowbTableKb / kRowbChunkKb)
+  static constexpr int ROWB_SLOTS = !ROWB_ ? 0 : PAIR_ ? kRowbChunks : 1;
+  static constexpr int ROWB_SLOT_BYTES = !ROWB_ ? 0 : PAIR_ ? kRowbChunkKb * BN_ * 4 : kRowbTableKb * BN_ * 4;
+  static constexpr int ROWB_BYTES = ROWB_SLOTS * ROWB_SLOT_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_STAGE_BYTES + ROWB_BYTES + BAR_BYTES + 1024;  // +1024: alignment slack
 };
 
 // Tile order: panels of kRasterGroup M-blocks; inside a panel the M index runs fastest, then
 // N. The 148 tiles in flight at any time then cover a roughly square patch of C, so the
 // A rows and B rows they share are fetched from DRAM once and hit in L2 afterwards.
 constexpr int kRasterGroup = 32;
-
-// Row-scaled kernel: K blocks of per-column B scales held in shared memory per tile (128 floats each).
-constexpr int kRowbTableKb = 64;
-constexpr int kRowbTableBytes = kRowbTableKb * 128 * 4;
 
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int& m_blk, int& n_blk,
                                             int group = kRasterGroup) {
@@ -280,26 +290,28 @@ template <int BN, bool MULTI, int SK, bool MC = false, bool ROWB = false, int A_
 __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b,
                                                const GemmArgs& args, const CUtensorMap* dmaps,
                                                const CUtensorMap* tmap_bst = nullptr) {
-  using Cfg = TileCfg<BN, MULTI, A_ROWS, PAIR>;
+  using Cfg = TileCfg<BN, MULTI, A_ROWS, PAIR, ROWB>;
   constexpr int STAGES = Cfg::STAGES;
   constexpr uint32_t TS = Cfg::TMEM_STAGES;
   constexpr uint32_t H = Cfg::HALVES;
-  static_assert(!(PAIR && (MC || ROWB)), "pair kernels: block scales, plain or TMA-store output");
+  static_assert(!(PAIR && MC), "pair kernels: plain or TMA-store output");
+  static_assert(!(PAIR == 1 && ROWB), "row-scaled B: the split pair form only");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* out_stage = smem + STAGES * Cfg::STAGE_BYTES;
-  static_assert(!(ROWB && MULTI), "the row-scaled kernel has one destination");
-  float* rowb_table = reinterpret_cast<float*>(out_stage);   // ROWB: [kRowbTableKb][128] B scales of the current tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + (ROWB ? kRowbTableBytes : Cfg::OUT_STAGE_BYTES));
+  // ROWB: B scales, [kRowbTableKb][128] of the current tile, or kRowbChunks x [kRowbChunkKb][256] (pairs)
+  float* rowb_table = reinterpret_cast<float*>(out_stage + Cfg::OUT_STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + Cfg::OUT_STAGE_BYTES + Cfg::ROWB_BYTES);
+  constexpr int SLOTS = Cfg::ROWB_SLOTS > 0 ? Cfg::ROWB_SLOTS : 1;
   uint64_t* full = bars;                  // [STAGES]  TMA bytes landed
   uint64_t* empty = bars + STAGES;        // [STAGES]  MMA finished reading the slot
   uint64_t* tfull = bars + 2 * STAGES;    // [TS * H]  TMEM stage (half) holds a finished K-block partial
   uint64_t* tempty = bars + 2 * STAGES + TS * H;  // [TS * H]  every epilogue warp has read the TMEM stage (half)
-  uint64_t* sfull = bars + 2 * STAGES + 2 * TS * H;     // ROWB: the tile's scale table has landed
-  uint64_t* sempty = sfull + 1;                           // ROWB: every promotion warp is done with the table
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * TS * H + 2);
-  static_assert((2 * STAGES + 2 * TS * H + 2) * 8 + 8 <= Cfg::BAR_BYTES, "barrier area too small");
+  uint64_t* sfull = bars + 2 * STAGES + 2 * TS * H;     // [SLOTS] ROWB: the scale table (chunk) has landed
+  uint64_t* sempty = sfull + SLOTS;                       // [SLOTS] ROWB: every promotion warp is done with it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * TS * H + 2 * SLOTS);
+  static_assert((2 * STAGES + 2 * TS * H + 2 * SLOTS) * 8 + 8 <= Cfg::BAR_BYTES, "barrier area too small");
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5;
@@ -325,8 +337,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], PAIR ? 2 * (Cfg::EPI_WARPS / H) : (Cfg::EPI_WARPS / 4) * live_quarters);
     }
-    mbar_init(sfull, 1);
-    mbar_init(sempty, (Cfg::EPI_WARPS / 4) * live_quarters);
+    for (int s = 0; s < SLOTS; ++s) {
+      mbar_init(&sfull[s], 1);
+      mbar_init(&sempty[s], (Cfg::EPI_WARPS / 4) * live_quarters);
+    }
     *abort_flag = 0u;
     fence_barrier_init();
   }
@@ -369,10 +383,11 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       bool a_pending = args.a_from_prep != 0;
       if constexpr (PAIR) {
         // (pair kernels are not the decode path: they simply wait before their first load)
-        if (a_pending) asm volatile("griddepcontrol.wait;" ::: "memory");
+        // (ROWB: the scale chunks come from the prep launch too)
+        if (a_pending || ROWB) asm volatile("griddepcontrol.wait;" ::: "memory");
         a_pending = false;
       }
-      uint32_t tile_no = 0;
+      uint32_t tile_no = 0;   // ROWB: scale tables (pairs: chunks) loaded so far
       (void)tile_no;
       uint32_t pend_from = 0;
       int pend_kb0 = 0, pend_m0 = 0;
@@ -387,7 +402,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       while (ok && seg_next<SK>(cur, args, num_m, num_n, num_kb, num_tiles, seg)) {
         const int m0 = seg.m_blk * Cfg::TILE_M + static_cast<int>(cta_rank) * Cfg::BM;
         const int n0 = seg.n_blk * BN;
-        if constexpr (ROWB) {
+        if constexpr (ROWB && !PAIR) {
           if (args.rowb_table) {
             // the B scales of this tile: one box [K blocks x 128 columns] of the K-block-major copy, once
             // the promotion warps have let go of the previous tile's table
@@ -399,6 +414,17 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
           }
         }
         for (int kb = seg.kb_begin; kb < seg.kb_end; ++kb, ++it) {
+          if constexpr (ROWB && PAIR) {
+            if ((kb - seg.kb_begin) % kRowbChunkKb == 0) {
+              // the next chunk of B scales: one box [8 K blocks x 256 columns] of the K-block-major copy (zeros
+              // beyond its edges), once the promotion warps of this CTA have let go of the chunk three before
+              const uint32_t c = tile_no % SLOTS;
+              if (!mbar_wait(&sempty[c], ((tile_no / SLOTS) & 1u) ^ 1u, abort_flag, status_word)) { ok = false; break; }
+              mbar_arrive_expect_tx(&sfull[c], Cfg::ROWB_SLOT_BYTES);
+              tma_load_2d(rowb_table + c * (Cfg::ROWB_SLOT_BYTES / 4), tmap_bst, &sfull[c], n0, kb);
+              ++tile_no;
+            }
+          }
           const uint32_t s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
           if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, status_word)) { ok = false; break; }
@@ -442,6 +468,18 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
               asm volatile("griddepcontrol.wait;" ::: "memory");
               a_pending = false;
               for (uint32_t j = pend_from; j <= it; ++j) load_a(j % STAGES, pend_kb0 + static_cast<int>(j - pend_from), pend_m0);
+            }
+          }
+        }
+      }
+      if constexpr (ROWB && PAIR) {
+        // Abort path: the scale chunks are this CTA's own copies, whichever rank it has
+        if (!ok) {
+          const uint32_t first = tile_no > static_cast<uint32_t>(SLOTS) ? tile_no - SLOTS : 0u;
+          for (uint32_t j = first; j < tile_no; ++j) {
+            const uint64_t t0 = globaltimer_ns();
+            while (!mbar_try_wait(&sfull[j % SLOTS], (j / SLOTS) & 1u)) {
+              if (globaltimer_ns() - t0 > kWaitLimitNs) break;
             }
           }
         }
@@ -548,7 +586,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
     uint32_t it = 0;
     uint32_t out_pass = 0;     // boxes this warp has staged so far (picks the staging buffer)
     (void)out_pass;
-    uint32_t rowb_tile = 0;
+    uint32_t rowb_tile = 0;    // ROWB: scale tables (pairs: chunks) used so far
     (void)rowb_tile;
     bool ok = (warp & 3) < live_quarters;
     // the scale copy AsT is written by the preceding tile_prep_kernel; with programmatic
@@ -577,7 +615,9 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       nb = nb < num_nb ? nb : num_nb - 1;
       // lanes of a warp own consecutive rows: K-block-major scales make this one coalesced
       // 128-byte load per warp and K block (row-major As would be 32 separate sectors)
-      const float* as_col = args.AsT + row;
+      // (pair tiles of an odd last row block reach beyond the padded rows: those lanes read the last padded one, and
+      // nothing of theirs is stored)
+      const float* as_col = args.AsT + (row < args.m_pad ? row : args.m_pad - 1);
       const float* bs_row = args.Bs + static_cast<int64_t>(nb) * args.ld_bs;
 
       // accumulators as 32-column groups of pairs: acc[g][j] = columns 32 g + 2 j, + 1
@@ -592,7 +632,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       // bytes from the K-block-major copy) before the wait for the MMA, so that they arrive
       // while the warp waits; then acc += p * (sa * sb[col]) costs a multiply and an FMA.
       auto promote_rowb = [&](float sa, const float* sbt, bool from_smem) -> bool {
-        static_assert(!ROWB || CHUNKS == 2, "row-scaled B is built for the 128-wide tile only");
+        static_assert(!ROWB || PAIR || CHUNKS == 2, "row-scaled B: 128-wide tiles, or CTA pairs");
         float4 sv[16];
         if (from_smem) {
 #pragma unroll
@@ -626,6 +666,40 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
             // two columns at a time: (sa * s_lo, sa * s_hi) and the accumulation are one packed instruction each
             ffma2(acc[g & (CHUNKS - 1)][j], g ? pb[2 * j] : pa[2 * j], g ? pb[2 * j + 1] : pa[2 * j + 1],
                   fmul2_bcast(s_lo, s_hi, sa));
+          }
+        }
+        return true;
+      };
+
+      // The same on a CTA pair: 128 columns per thread, two 64-column TMEM loads, a few of the scales fetched
+      // ahead of each wait and the others between the multiplies. Bound by the shared-memory port: 128 broadcast
+      // floats per warp and K block (~600 clocks for the eight warps) beside 256 of TMA fill and 256 of operand
+      // reads; per output element that is the same fetch as on the 128-wide tile, with half of the fill and
+      // of the operand reads. 4096 x 4096 x 8192: 222 us against 269 us on 128 x 128 tiles.
+      auto promote_rowb_pair = [&](float sa, const float* sbt) -> bool {
+        const float4* s4p = reinterpret_cast<const float4*>(sbt);
+        const uint32_t ts = it % TS;
+        const uint32_t tph = (it / TS) & 1u;
+        ++it;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[ts * H + hb], tph, abort_flag, status_word))) return false;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + lane_col + ts * BN;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t p[64];
+          tmem_ld_32x64(taddr + half * 64, p);
+          float4 pre[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) pre[i] = s4p[half * 16 + i];
+          tmem_ld_wait_64(p);
+          if (half == 1) release_stage(ts * H + hb);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {   // columns 64 half + 4 i .. + 3
+            const float4 s4 = i < 2 ? pre[i & 1] : s4p[half * 16 + i];
+            const int g = (2 * half + (i >> 3)) % CHUNKS;
+            const int j = (2 * i) & 15;
+            ffma2(acc[g][j], p[4 * i], p[4 * i + 1], fmul2_bcast(s4.x, s4.y, sa));
+            ffma2(acc[g][j + 1], p[4 * i + 2], p[4 * i + 3], fmul2_bcast(s4.z, s4.w, sa));
           }
         }
         return true;
@@ -678,13 +752,13 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       // The scales AsT[kb][row] and Bs[nb, kb] come from global memory (L2 latency of several
       // hundred clocks). They are fetched a whole group of PF K blocks ahead so that their
       // first use never stalls the promotion loop.
-      if constexpr (ROWB) {
+      if constexpr (ROWB && !PAIR) {
         if (args.rowb_table) {
           ok = __all_sync(0xffffffffu, mbar_wait(sfull, rowb_tile & 1u, abort_flag, status_word));
           if (!ok) break;
         }
       }
-      constexpr int PF = (CHUNKS == 2) ? 2 : 4;
+      constexpr int PF = (CHUNKS == 2 || ROWB) ? 2 : 4;
       float sa_c[PF], sb_c[PF], sa_n[PF], sb_n[PF];
       const int kb_last = seg.kb_end - 1;
 #pragma unroll
@@ -704,7 +778,19 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
 #pragma unroll
         for (int j = 0; j < PF; ++j) {
           if (ok && kb0 + j < seg.kb_end) {
-            if constexpr (ROWB) {
+            if constexpr (ROWB && PAIR) {
+              const int rel = kb0 + j - seg.kb_begin;
+              const uint32_t c = rowb_tile % SLOTS;
+              if (rel % kRowbChunkKb == 0)
+                ok = __all_sync(0xffffffffu, mbar_wait(&sfull[c], (rowb_tile / SLOTS) & 1u, abort_flag, status_word));
+              if (ok) ok = promote_rowb_pair(sa_c[j], rowb_table + (c * kRowbChunkKb + rel % kRowbChunkKb) * BN + cw * Cfg::EPI_COLS);
+              if (ok && (rel % kRowbChunkKb == kRowbChunkKb - 1 || kb0 + j + 1 == seg.kb_end)) {
+                // done with this chunk: the producer may load another into its slot
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sempty[c]);
+                ++rowb_tile;
+              }
+            } else if constexpr (ROWB) {
               ok = args.rowb_table
                        ? promote_rowb(sa_c[j], rowb_table + (kb0 + j) * 128 + cw * Cfg::EPI_COLS, true)
                        : promote_rowb(sa_c[j], args.BsT + static_cast<int64_t>(kb0 + j) * args.n_pad + col0, false);
@@ -720,7 +806,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
         }
       }
       if (!ok) break;
-      if constexpr (ROWB) {
+      if constexpr (ROWB && !PAIR) {
         if (args.rowb_table) {
           // done with this tile's scale table: the producer may load the next one
           __syncwarp();
@@ -947,6 +1033,15 @@ __global__ void __launch_bounds__(TileCfg<BN, false>::THREADS, 1)
 gemm_tile_rowb_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_bst, const GemmArgs args) {
   gemm_tile_body<BN, false, 0, false, true>(tmap_a, tmap_b, args, nullptr, &tmap_bst);
+}
+
+// Row-scaled B on CTA pairs (the split form, staged output), without and with the split-K tail.
+template <int SK>
+__global__ void __launch_bounds__(TileCfg<256, true>::THREADS, 1)
+gemm_pair_rowb_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                      const __grid_constant__ CUtensorMap tmap_bst, const GemmArgs args,
+                      const __grid_constant__ DstMaps dmaps) {
+  gemm_tile_body<256, true, SK, false, true, 128, 2>(tmap_a, tmap_b, args, dmaps.m, &tmap_bst);
 }
 
 // Multicast form: args.dst[0] is a multimem address; every 128-byte row segment of a finished

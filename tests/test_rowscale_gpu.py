@@ -79,3 +79,22 @@ def test_legacy_call_form_of_the_reference_harness(device):
     assert oracle.max_err_over_rms(out.cpu(), oracle.gemm_rowscale_dequant(A, B, As, Bs)) <= 1e-4
     out16 = pkg.w8a8_block_fp8_matmul(*d, 128, torch.bfloat16)
     assert torch.equal(out16, deep_gemm.gemm_fp8_fp8_bf16_nt(*d, 128))
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 128), (257, 1100, 1152), (512, 4104, 1040), (1000, 9472, 2064), (2100, 2304, 640),
+                                   (256, 4096, 4096), (1000, 3008, 4112)])
+def test_rowscale_on_cta_pairs(device, M, N, K):
+    """Sizes at which the 256 x 256 form runs or borders on: odd numbers of 128-row blocks, columns and K blocks that fill no
+    tile and no scale chunk (8 K blocks), rows that are not 16-byte multiples (register stores, 128 x 128 tiles), whole
+    waves, a last wave split along K whose ranges start inside a chunk, chunks recycled over several tiles."""
+    A, B, As, Bs = oracle.make_rowscale_inputs(M, N, K, M + N + K)
+    d = [t.to(device) for t in (A, B, As, Bs)]
+    a = (d[0].double() * d[2].double().repeat_interleave(128, 1)[:, :K])
+    ref = a @ (d[1].double() * d[3].double().repeat_interleave(128, 1)[:, :K]).T
+    out32 = runtime.gemm_rowscale(*d, 128, torch.float32)
+    # fp32 accumulation over K blocks, exact fp32 products inside one: a few roundings of 2^-24 each per K block
+    rel = ((out32.double() - ref).norm() / ref.norm()).item()
+    assert rel <= 2.0 ** -24 * (2 + -(-K // 128)) ** 0.5 * 4
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.float32), out32)
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.bfloat16), out32.to(torch.bfloat16))
+    runtime.check_device_status()
