@@ -25,6 +25,7 @@ struct DeviceInfo {
   int cc_major = 0;
   int sm_count = 0;
   int pair_clusters = 0;   // CTA pairs of the pair kernels that can be resident at once
+  int clusters[kClusterMax + 1] = {};   // clusters of c CTAs of gemm_cluster_kernel that can be resident at once
 };
 DeviceInfo g_dev[kMaxDevices];
 std::mutex g_mutex;
@@ -64,6 +65,9 @@ int device_info(const DeviceInfo** out) {
               128 * StreamKCfg<256>::REGS_CONTROL + 256 * StreamKCfg<256>::REGS_EPILOGUE);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_kernel<128, 0>), TileCfg<128, false>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_kernel<256, 0>), TileCfg<256, false>::SMEM_BYTES);
+      opt_in(reinterpret_cast<const void*>(&gemm_cluster_kernel), TileCfg<128, false>::SMEM_BYTES);
+      regs_ok(reinterpret_cast<const void*>(&gemm_cluster_kernel), TileCfg<128>::THREADS,
+              128 * TileCfg<128>::REGS_CONTROL + 256 * TileCfg<128>::REGS_EPILOGUE);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_multi_kernel<128>), TileCfg<128, true>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_multi_kernel<256>), TileCfg<256, true>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_rowb_kernel<128>), TileCfg<128, false, 128, 0, true>::SMEM_BYTES);
@@ -131,6 +135,17 @@ int device_info(const DeviceInfo** out) {
           n_clusters = 0;
         }
         d.pair_clusters = n_clusters < d.sm_count / 2 ? n_clusters : d.sm_count / 2;
+        ccfg.blockDim = dim3(TileCfg<128>::THREADS);
+        ccfg.dynamicSmemBytes = TileCfg<128, false>::SMEM_BYTES;
+        for (int c = 2; c <= kClusterMax; ++c) {
+          cattr[0].val.clusterDim.x = static_cast<unsigned>(c);
+          ccfg.gridDim = dim3(static_cast<unsigned>(d.sm_count / c * c));
+          if (cudaOccupancyMaxActiveClusters(&n_clusters, gemm_cluster_kernel, &ccfg) != cudaSuccess) {
+            cudaGetLastError();
+            n_clusters = 0;
+          }
+          d.clusters[c] = n_clusters < d.sm_count / c ? n_clusters : d.sm_count / c;
+        }
       }
       opt_in(reinterpret_cast<const void*>(&gemm_streamk_kernel<16>), StreamKCfg<16>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_streamk_kernel<32>), StreamKCfg<32>::SMEM_BYTES);
@@ -348,47 +363,76 @@ TileSkPlan pair_sk_plan(int64_t M, int64_t N, int64_t K, int pairs) {
   return p;
 }
 
-double wave_efficiency(int64_t tiles, int sms) {
-  if (tiles <= 0) return 1.0;
-  const int64_t waves = (tiles + sms - 1) / sms;
-  return static_cast<double>(tiles) / static_cast<double>(waves * sms);
+// AUTO's estimate of each form's time in us, fitted to graph replays of 46 shapes with 129..8192 rows, 512..28672 columns
+// and 1024..8192 deep (single launches on B200): a start-up, then per wave of tiles the K blocks at the form's rate
+// and the end of a tile (register stores in the split single-CTA form, staged ones otherwise), and 6 us for the
+// fix-up pass of a split last wave. Its choice is 1.5 % slower than the fastest form of each shape in the mean; the rule
+// before it (wave efficiencies, an even number of row blocks for CTA pairs) was 11.5 % slower. For instance, measured
+// 128 x 128 / 128 x 256 / its split tail / pairs / their split tail: 1611 x 7000 x 4208 79.5 / 69.9 / 70.8 / 57.7 / 57.5,
+// 2545 x 1920 x 6272 64.1 / 54.0 / 44.3 / 53.4 / 42.7, 317 x 24832 x 2432 41.9 / 27.6 / 28.2 / 36.5 / 36.5,
+// 1394 x 1536 x 1152 10.7 / 11.1 / 14.8 / 11.1 / 16.0, 4096 x 4096 x 8192 184.3 / 149.3 / 143.2 / 151.6 / 135.0.
+struct Pick {
+  int variant;
+  double us;
+};
+
+double split_waves_us(const TileSkPlan& p, int workers, double per_kb, double per_tile) {
+  return (p.full / workers) * (per_kb * p.num_kb + per_tile) + per_kb * p.kb_per + per_tile + 6.0;
 }
 
-int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
+Pick pick_form(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   const bool pair_ok = pairs > 0;
+  const double kb = static_cast<double>((K + 127) / 128);
+  const int64_t num_m = (M + 127) / 128;
+  auto waves = [](int64_t tiles, int64_t workers) { return static_cast<double>((tiles + workers - 1) / workers); };
   // Decode shapes (M <= 256) are weight-streaming and HBM-bound. Measured on B200 at N = 28672,
   // K = 8192: the plain 128x256 tile kernel (46 us at M = 16, 5.1 TB/s with 112 of 148 SMs busy)
   // beats the swap-AB stream-K kernel (65 us), so AUTO does not pick that one.
   // (two row blocks, M in 129..256, go to the CTA pairs below when the device runs them: 79.5 vs 84-86 us at M = 256)
-  if (M <= 128 || (M <= 256 && (N <= 128 || !pair_ok)))
-    return (N > 128) ? B200FP8_VARIANT_TILE256 : B200FP8_VARIANT_TILE128;
-  const int64_t num_m = (M + 127) / 128;
-  const double e128 = wave_efficiency(num_m * ((N + 127) / 128), sm_count);
-  const double e256 = wave_efficiency(num_m * ((N + 255) / 256), sm_count);
-  // the 128x256 tile moves 25 % fewer operand bytes per flop; prefer it unless the last wave is much emptier
-  if (e256 * 1.15 < e128) return B200FP8_VARIANT_TILE128;
-  // CTA pairs on 256 x 256 tiles with the output staged through shared memory and written by TMA
-  // (two staging sets per warp): the same tile waves as the single-CTA form when the number of
-  // M-blocks is even, and measured faster than it and than its tail split-K form (8192 x 18432 x 7168:
-  // 1.034 vs 1.11 ms, 1790 vs 1674 TFLOP/s sustained over 2.4 s; 4096 x 4096 x 8192: 141.3 vs 145.3 us).
-  // With the stores out of the way the form that issues each K block as two 128-column halves is the
-  // faster of the two pair kernels (same shapes: 1.002 vs 1.016 ms, 1846 vs 1811 sustained; 136.2 vs 139.4 us).
-  if (pair_ok && num_m % 2 == 0) {
-    // a partly empty last wave of pair tiles is split along K. The pair form's whole-tile part is not slower
-    // for it and the fix-up pass is a few microseconds, so the bar is low: the idle share of the last wave
-    // at least a fiftieth of the run (8192 x 18432 x 7168, 10 tiles in the 32nd wave: 986-989 vs 999-1000 us)
-    const TileSkPlan pp = pair_sk_plan(M, N, K, pairs);
-    const int64_t pw = (static_cast<int64_t>(pp.num_m) * pp.num_n + pairs - 1) / pairs;
-    const bool pworth = pp.split >= 2 && (1.0 - 1.0 / pp.split) >= 0.02 * static_cast<double>(pw);
-    return pworth ? B200FP8_VARIANT_PAIR256_SPLIT_SK : B200FP8_VARIANT_PAIR256_SPLIT;
+  if (M <= 128 || (M <= 256 && (N <= 128 || !pair_ok))) {
+    const int64_t bn = N > 128 ? 256 : 128;
+    return {N > 128 ? B200FP8_VARIANT_TILE256 : B200FP8_VARIANT_TILE128,
+            6.0 + 0.43 * kb * waves(num_m * ((N + bn - 1) / bn), sm_count)};
   }
-  // A mostly empty last wave is worth splitting along K, but the split-K kernel runs its
-  // whole-tile part about 5 % slower (measured) and adds a fix-up pass: only take it when the
-  // idle share of the last wave is at least a tenth of the whole run.
-  const TileSkPlan p = tile_sk_plan(M, N, K, sm_count);
-  const int64_t waves = (static_cast<int64_t>(p.num_m) * p.num_n + sm_count - 1) / sm_count;
-  const bool worth = p.split >= 2 && (1.0 - 1.0 / p.split) >= 0.10 * static_cast<double>(waves);
-  return worth ? B200FP8_VARIANT_TILE256_SK : B200FP8_VARIANT_TILE256;
+  Pick best = {B200FP8_VARIANT_TILE128, 6.0 + waves(num_m * ((N + 127) / 128), sm_count) * (0.405 * kb + 0.5)};
+  auto consider = [&best](int variant, double us) {
+    if (us < best.us) best = {variant, us};
+  };
+  const TileSkPlan t = tile_sk_plan(M, N, K, sm_count);
+  consider(B200FP8_VARIANT_TILE256, 5.0 + waves(static_cast<int64_t>(t.num_m) * t.num_n, sm_count) * (0.52 * kb + 1.3));
+  if (t.split >= 2) consider(B200FP8_VARIANT_TILE256_SK, 5.0 + split_waves_us(t, sm_count, 0.54, 2.5));
+  if (pair_ok) {
+    const TileSkPlan p = pair_sk_plan(M, N, K, pairs);
+    consider(B200FP8_VARIANT_PAIR256_SPLIT, 5.3 + waves(static_cast<int64_t>(p.num_m) * p.num_n, pairs) * (0.50 * kb + 1.3));
+    if (p.split >= 2) consider(B200FP8_VARIANT_PAIR256_SPLIT_SK, 5.3 + split_waves_us(p, pairs, 0.50, 1.3));
+  }
+  return best;
+}
+
+int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
+  return pick_form(M, N, K, sm_count, pairs).variant;
+}
+
+// CTAs per tile (2..8) for products whose 128 x 128 tiles leave SMs idle: the K blocks of a tile are cut over a cluster
+// (gemm_cluster_kernel), as far as all clusters are resident at once. 1: another form is estimated to be faster.
+// Cutting costs about 2 us (two cluster barriers and the addition through distributed shared memory), so that products of
+// fewer than 12 K blocks stay whole. Measured, one / two / four CTAs per tile, us: 4 x 2560 x 2048 12.9 / 9.0 / 8.1,
+// 64 x 2048 x 4096 20.1 / 12.3 / 9.4, 512 x 512 x 2048 11.4 / 11.3 / 9.2, 512 x 512 x 8192 28.9 / 19.5 / 13.3,
+// 1 x 8192 x 8192 34.0 / 17.6 / - (more clusters than fit: 22.3).
+int cluster_split(int64_t M, int64_t N, int64_t K, const int* clusters, double other_us) {
+  const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
+  const int64_t kblocks = (K + 127) / 128;
+  int best = 1;
+  if (kblocks < 12) return best;
+  for (int c = 2; c <= kClusterMax; ++c) {
+    if (tiles > clusters[c] || kblocks < 2 * c) continue;
+    const double us = 8.2 + 0.405 * static_cast<double>((kblocks + c - 1) / c);
+    if (us < other_us) {
+      other_us = us;
+      best = c;
+    }
+  }
+  return best;
 }
 
 // Row-scaled B: 128 x 128 tiles, or 256 x 256 tiles on CTA pairs (with the last wave split along K where that can be
@@ -412,7 +456,7 @@ int pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
 
 template <int BN>
 int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda, int64_t ldb, int sm_count,
-                cudaStream_t stream, int64_t sk_grid = 0) {
+                cudaStream_t stream, int64_t sk_grid = 0, int cluster = 1) {
   CUtensorMap ta, tb;
   // Weight-streaming shapes: kernel forms with 16- or 64-row A slots and six or five pipeline stages
   // (measured 3-4 % faster than the 128-row form at N = 28672, K = 8192: 44.5-46 us at M <= 17).
@@ -429,9 +473,13 @@ int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda,
   const int grid = sk_grid > 0 ? static_cast<int>(sk_grid) : static_cast<int>(tiles < sm_count ? tiles : sm_count);
   // Programmatic dependent launch: the kernel may begin (barrier set-up, TMEM allocation,
   // operand loads) while the tile_prep_kernel enqueued just before it is still running.
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(TileCfg<BN, false>::THREADS);
@@ -439,7 +487,12 @@ int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda,
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t err;
-  if (decode && a_rows == 16u) {
+  if (BN == 128 && cluster > 1) {
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
+    cfg.numAttrs = 2;
+    cfg.dynamicSmemBytes = TileCfg<128, false>::SMEM_BYTES;
+    err = cudaLaunchKernelEx(&cfg, gemm_cluster_kernel, ta, tb, args);
+  } else if (decode && a_rows == 16u) {
     cfg.dynamicSmemBytes = TileCfg<256, false, 16>::SMEM_BYTES;
     err = cudaLaunchKernelEx(&cfg, gemm_tile_decode_kernel<256, 16>, ta, tb, args);
   } else if (decode) {
@@ -771,7 +824,12 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
 
   const bool auto_variant = variant == B200FP8_VARIANT_AUTO;
   // (the pair form only pays with the staged output: a destination that cannot take 16-byte rows gets the single-CTA choice)
-  if (auto_variant) variant = pick_variant(M, N, K, dev->sm_count, (staged && !mc && !fq.rowb) ? dev->pair_clusters : 0);
+  double auto_us = 0.0;
+  if (auto_variant) {
+    const Pick p = pick_form(M, N, K, dev->sm_count, (staged && !mc && !fq.rowb) ? dev->pair_clusters : 0);
+    variant = p.variant;
+    auto_us = p.us;
+  }
   if (fq.rowb) {
     variant = pick_rowb(M, N, K, dev->sm_count, staged ? dev->pair_clusters : 0);
     // (a workspace without room for the partial tiles: the same tiles without the split tail)
@@ -781,6 +839,8 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       variant = B200FP8_VARIANT_PAIR256_SPLIT;
   }
   const bool multi = n_dst > 1 || mc;
+  const int cluster = auto_variant && !multi && !fq.rowb ? cluster_split(M, N, K, dev->clusters, auto_us) : 1;
+  if (cluster > 1) variant = B200FP8_VARIANT_TILE128;
   if (fq.rowb && (multi || fused_q)) return B200FP8_ERR_VARIANT;
   // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room
   // for a second set of output staging buffers, which keeps NVLink busy through the next tile's K loop
@@ -895,7 +955,8 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       return launch_pair<false>(a_eff, B, args, lda_eff, ldb, dev->pair_clusters, stream);
     if (variant == B200FP8_VARIANT_PAIR256_SPLIT)
       return launch_pair<true>(a_eff, B, args, lda_eff, ldb, dev->pair_clusters, stream);
-    return variant == B200FP8_VARIANT_TILE128 ? launch_tile<128>(a_eff, B, args, lda_eff, ldb, dev->sm_count, stream)
+    return variant == B200FP8_VARIANT_TILE128
+               ? launch_tile<128>(a_eff, B, args, lda_eff, ldb, dev->sm_count, stream, 0, cluster)
                                               : launch_tile<256>(a_eff, B, args, lda_eff, ldb, dev->sm_count, stream);
   }
 

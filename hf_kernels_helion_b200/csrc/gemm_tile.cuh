@@ -276,17 +276,87 @@ __device__ __forceinline__ bool seg_next(SegCursor& c, const GemmArgs& a, int nu
   return false;
 }
 
+// K range of one CTA of a cluster that shares a tile (CL kernels): even cuts, in rank order.
+__device__ __forceinline__ void cluster_range(int rank, int size, int num_kb, int& kb_begin, int& kb_end) {
+  kb_begin = static_cast<int>(static_cast<int64_t>(rank) * num_kb / size);
+  kb_end = static_cast<int>(static_cast<int64_t>(rank + 1) * num_kb / size);
+}
+
 // Tensor maps of the destinations of the multi-destination kernel: byte matrices
 // [M rows, N * element size] with box 32 rows x 128 bytes, SWIZZLE_128B.
 struct DstMaps {
   CUtensorMap m[8];
 };
 
+// CL kernels, after the K loops: CTA `rank` of the cluster owns every size-th row of the tile, adds the partial tiles
+// of all ranks in rank order (a fixed order: bit-reproducible) and writes the rows out, a warp per row and 128
+// columns, so that a row leaves as 256 (bf16) or 512 (fp32) contiguous bytes. Pitch of a partial tile: 132 floats, which
+// keeps both the row-per-lane writes and the row-wise reads free of bank conflicts. Warps 4..11.
+constexpr int kClusterPitch = 132;
+constexpr int kClusterMax = 8;   // the portable cluster size
+static_assert(128 * kClusterPitch * 4 <= TileCfg<128>::STAGES * TileCfg<128>::STAGE_BYTES, "the operand ring holds a partial tile");
+
+__device__ __forceinline__ void cluster_reduce_store(const GemmArgs& args, const uint8_t* smem, int tile, int num_m,
+                                                     int num_n, int rank, int size) {
+  int m_blk, n_blk;
+  tile_coords(tile, num_m, num_n, m_blk, n_blk);
+  const int w = static_cast<int>(threadIdx.x >> 5) - 4;
+  const int lane = static_cast<int>(threadIdx.x & 31);
+  const int64_t left = args.M - static_cast<int64_t>(m_blk) * 128;
+  const int rows = left < 128 ? static_cast<int>(left) : 128;
+  const int64_t col = static_cast<int64_t>(n_blk) * 128 + lane * 4;
+  const uint32_t base = smem_u32(smem) + lane * 16;
+  for (int r = rank + w * size; r < rows; r += 8 * size) {
+    float4 v[kClusterMax];   // all ranks' loads are in flight together
+#pragma unroll
+    for (int j = 0; j < kClusterMax; ++j)
+      if (j < size) v[j] = ld_shared_cluster_v4(mapa_shared(base + r * (kClusterPitch * 4), static_cast<uint32_t>(j)));
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kClusterMax; ++j) {
+      if (j < size) {
+        sum.x += v[j].x;
+        sum.y += v[j].y;
+        sum.z += v[j].z;
+        sum.w += v[j].w;
+      }
+    }
+    const int64_t row = static_cast<int64_t>(m_blk) * 128 + r;
+    if (args.out_fp32) {
+      float* c = reinterpret_cast<float*>(args.C) + row * args.ldc + col;
+      if (col + 4 <= args.N && (reinterpret_cast<uintptr_t>(c) & 15u) == 0) {
+        *reinterpret_cast<float4*>(c) = sum;
+      } else {
+        if (col < args.N) c[0] = sum.x;
+        if (col + 1 < args.N) c[1] = sum.y;
+        if (col + 2 < args.N) c[2] = sum.z;
+        if (col + 3 < args.N) c[3] = sum.w;
+      }
+    } else {
+      __nv_bfloat16* c = reinterpret_cast<__nv_bfloat16*>(args.C) + row * args.ldc + col;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(sum.x, sum.y), hi = __floats2bfloat162_rn(sum.z, sum.w);
+      if (col + 4 <= args.N && (reinterpret_cast<uintptr_t>(c) & 7u) == 0) {
+        uint2 u;
+        u.x = *reinterpret_cast<const uint32_t*>(&lo);
+        u.y = *reinterpret_cast<const uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>(c) = u;
+      } else {
+        if (col < args.N) c[0] = lo.x;
+        if (col + 1 < args.N) c[1] = lo.y;
+        if (col + 2 < args.N) c[2] = hi.x;
+        if (col + 3 < args.N) c[3] = hi.y;
+      }
+    }
+  }
+}
+
 // MULTI: the result leaves through the shared-memory staging area; MC (with MULTI): by
 // multimem.st to a multicast address, otherwise by TMA stores to up to eight destinations.
 // ROWB: B carries one scale per ROW and K block (the deep-gemm layout) instead of one per
 // 128 x 128 block: the promotion multiplies every accumulator column by its own scale.
-template <int BN, bool MULTI, int SK, bool MC = false, bool ROWB = false, int A_ROWS = 128, int PAIR = 0>
+// CL: the CTAs of a cluster share ONE tile, each with its range of K blocks; the partial sums meet through
+// distributed shared memory (see cluster_reduce_store) and no CTA has a second tile.
+template <int BN, bool MULTI, int SK, bool MC = false, bool ROWB = false, int A_ROWS = 128, int PAIR = 0, bool CL = false>
 __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b,
                                                const GemmArgs& args, const CUtensorMap* dmaps,
                                                const CUtensorMap* tmap_bst = nullptr) {
@@ -296,6 +366,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
   constexpr uint32_t H = Cfg::HALVES;
   static_assert(!(PAIR && MC), "pair kernels: plain or TMA-store output");
   static_assert(!(PAIR == 1 && ROWB), "row-scaled B: the split pair form only");
+  static_assert(!CL || (!PAIR && !MULTI && !SK && !ROWB && BN == 128), "cluster split: plain 128-wide tiles");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -321,8 +392,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
   // promotion warps. `empty` and `tfull` exist in both CTAs and the leader signals each copy.
   const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;
   const bool leader = cta_rank == 0u;
-  const int worker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-  const int nworkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+  const int cl_size = CL ? static_cast<int>(cluster_nctarank()) : 1;
+  const int cl_rank = CL ? static_cast<int>(cluster_ctarank()) : 0;
+  const int worker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x) / cl_size;
+  const int nworkers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x) / cl_size;
   // With a single block of rows and fewer than 97 of them (decode shapes) the upper TMEM lane
   // quarters hold rows that do not exist: the promotion warps of those quarters have nothing to
   // do and sit the kernel out (fewer instructions issued, and fewer arrivals per TMEM stage).
@@ -368,6 +441,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
   const int num_kb = static_cast<int>((K + Cfg::BK - 1) / Cfg::BK);
   const int num_tiles = num_m * num_n;
   uint32_t* status_word = args.status_word;
+  // (CL: one tile per cluster, this CTA's K range of it)
+  auto cl_cut = [&](Segment& seg) {
+    if constexpr (CL) cluster_range(cl_rank, cl_size, num_kb, seg.kb_begin, seg.kb_end);
+  };
 
   if (warp < 4) {
     if constexpr (Cfg::REBALANCE_REGS) setmaxnreg_dec<Cfg::REGS_CONTROL>();
@@ -400,6 +477,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       Segment seg;
       const uint32_t full_leader = PAIR ? mapa_shared(smem_u32(full), 0u) : 0u;
       while (ok && seg_next<SK>(cur, args, num_m, num_n, num_kb, num_tiles, seg)) {
+        cl_cut(seg);
         const int m0 = seg.m_blk * Cfg::TILE_M + static_cast<int>(cta_rank) * Cfg::BM;
         const int n0 = seg.n_blk * BN;
         if constexpr (ROWB && !PAIR) {
@@ -516,7 +594,12 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
     uint32_t it = 0;
     uint32_t last = 0xffffffffu;
     bool ok = true;
-    const uint32_t total_it = seg_total_kblocks<SK>(args, worker, nworkers, num_m, num_n, num_kb, num_tiles);
+    uint32_t total_it = seg_total_kblocks<SK>(args, worker, nworkers, num_m, num_n, num_kb, num_tiles);
+    if constexpr (CL) {
+      Segment seg;
+      cl_cut(seg);
+      total_it = static_cast<uint32_t>(seg.kb_end - seg.kb_begin);
+    }
     {
       for (; it < total_it; ++it) {
         if ((it & 1u) != p) continue;
@@ -607,6 +690,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       if constexpr (PAIR) cur.group = kRasterGroup / 2;   // 256-row tiles: the same 4096 rows per panel
     Segment seg;
     while (ok && seg_next<SK>(cur, args, num_m, num_n, num_kb, num_tiles, seg)) {
+      cl_cut(seg);
       const int m0 = seg.m_blk * Cfg::TILE_M + static_cast<int>(cta_rank) * Cfg::BM;
       const int n0 = seg.n_blk * BN;
       const int64_t row = static_cast<int64_t>(m0) + q * 32 + lane;
@@ -816,7 +900,14 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       }
 
 #define ACC(i) (((i) & 1) ? acc[(i) >> 5][((i) & 31) >> 1].y : acc[(i) >> 5][((i) & 31) >> 1].x)
-      if (SK && (seg.kb_begin != 0 || seg.kb_end != num_kb)) {
+      if constexpr (CL) {
+        // All loads of this CTA have landed and all its MMAs have retired (this warp has waited for the last of
+        // both issuers): the operand ring is free and takes the partial tile.
+        float* prow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * kClusterPitch + cw * Cfg::EPI_COLS;
+#pragma unroll
+        for (int j = 0; j < Cfg::EPI_COLS; j += 4)
+          *reinterpret_cast<float4*>(prow + j) = make_float4(ACC(j), ACC(j + 1), ACC(j + 2), ACC(j + 3));
+      } else if (SK && (seg.kb_begin != 0 || seg.kb_end != num_kb)) {
         // tail split-K: this CTA saw only part of the K range - leave the fp32 partial sums of the
         // rows that exist in the workspace; tile_sk_fixup_kernel adds the ranges of the tile
         if (row < M) {
@@ -957,6 +1048,16 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
   }
 #undef ACC
 
+  if constexpr (CL) {
+    // every partial tile of the cluster is in shared memory; each CTA adds and stores its share of the rows;
+    // none leaves (or reuses its shared memory) before the others have read it
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 4) cluster_reduce_store(args, smem, worker, num_m, num_n, cl_rank, cl_size);
+    __syncwarp();
+    cluster_sync_all();
+  }
+
   // ------------------------------------------------------------------ teardown
   if constexpr (MULTI) {
     // the output copies of this warp must be complete (written) before the CTA exits
@@ -983,6 +1084,13 @@ __global__ void __launch_bounds__(TileCfg<BN, false>::THREADS, 1)
 gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const GemmArgs args) {
   gemm_tile_body<BN, false, SK>(tmap_a, tmap_b, args, nullptr);
+}
+
+// Cluster split (launch with a cluster dimension of 2, 4 or 8 that divides the grid; one tile per cluster).
+__global__ void __launch_bounds__(TileCfg<128, false>::THREADS, 1)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                    const GemmArgs args) {
+  gemm_tile_body<128, false, 0, false, false, 128, 0, true>(tmap_a, tmap_b, args, nullptr);
 }
 
 // CTA-pair forms (launch with cluster dimension 2 and an even grid): 256 x 256 tiles per pair.

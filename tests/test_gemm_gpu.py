@@ -352,3 +352,34 @@ def test_decode_forms_with_short_a_slots(device, M, N, K):
     assert oracle.bf16_ulp_error(big[:M].cpu(), ref) <= 1
     assert bool((big[M:] == 7.0).all())
     runtime.check_device_status()
+
+
+def _rel(out, A, B, As, Bs):
+    K = A.shape[1]
+    a = A.double() * As.double().repeat_interleave(128, 1)[:, :K]
+    b = B.double() * Bs.double().repeat_interleave(128, 1)[:, :K].repeat_interleave(128, 0)[:B.shape[0]]
+    ref = a @ b.T
+    return ((out.double() - ref).norm() / ref.norm()).item()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1536), (4, 2560, 2048), (16, 1280, 1552), (37, 700, 4208), (64, 1024, 8192),
+                                   (97, 201, 1664), (128, 512, 2048), (130, 384, 2048), (300, 900, 2992), (512, 512, 2048),
+                                   (1024, 1024, 8192), (1611, 2000, 1168), (2545, 1920, 6272)])
+def test_auto_on_small_and_ragged_products(device, M, N, K):
+    """Products whose tiles leave SMs idle run as clusters that share a tile (ranges of two K blocks and more, uneven ones, a
+    short last K block, rows and columns that fill no tile, rows of the result that are not 16-byte multiples); odd
+    numbers of row blocks run on CTA pairs. Into a view with sentinels around it, twice the same bits."""
+    A, B, As, Bs = _dev(oracle.make_quantised_inputs(M, N, K, M + N), device)
+    buf = torch.full((M + 2, N + 24), 7.0, dtype=torch.float32, device=device)
+    out32 = runtime.gemm(A, B, As, Bs, 128, 128, torch.float32, out=buf[1:M + 1, 8:8 + N])
+    # fp32 accumulation over K blocks, exact fp32 products inside one: a few roundings of 2^-24 each per K block
+    assert _rel(out32, A, B, As, Bs) <= 2.0 ** -24 * (2 + -(-K // 128)) ** 0.5 * 4
+    assert bool((buf[0] == 7).all()) and bool((buf[-1] == 7).all())
+    assert bool((buf[:, :8] == 7).all()) and bool((buf[:, 8 + N:] == 7).all())
+    assert torch.equal(runtime.gemm(A, B, As, Bs, 128, 128, torch.float32), out32)
+    # a bf16 view may have another alignment and with it another form: the same sums up to their order
+    half = torch.zeros(M, N + 3, dtype=torch.bfloat16, device=device)
+    out16 = runtime.gemm(A, B, As, Bs, 128, 128, torch.bfloat16, out=half[:, 1:N + 1])
+    assert _rel(out16, A, B, As, Bs) <= 2.0 ** -8
+    assert bool((half[:, 0] == 0).all()) and bool((half[:, N + 1:] == 0).all())
+    runtime.check_device_status()
