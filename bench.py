@@ -659,11 +659,11 @@ def main_ours(args):
                             "(each rank reads back its M/n_gpus row block of the assembled result); "
                             "read-back of step i overlaps upload + math of step i+1 (second stream); the quantised weight is a resident parameter; "
                             "phases_one_step_serial: one extra step with events between its phases and nothing overlapping, max over ranks, plus the pinned copies alone"},
-            # per step: quant_act_contig_kernel, tile_prep_kernel, the GEMM kernel; N > 1 adds the exchange's
-            # barrier kernel (fused) or NCCL's all-gather plus the slot -> [M,N] copy (not counted: not ours)
-            # per step: quantiser, scale re-layout, GEMM; + the split-K fix-up pass where AUTO takes such a form;
-            # + the barrier kernel of the fused exchange
-            "gpu_launches": steps * (3 + (1 if variant in (4, 7) and world == 1 else 0)
+            # per step: quantiser, GEMM; + the scale re-layout where the GEMM writes to several GPUs; + the split-K fix-up
+            # pass where AUTO takes such a form; + the barrier kernel of the fused exchange (NCCL's all-gather and the
+            # slot -> [M,N] copy are not counted: not ours)
+            "gpu_launches": steps * (2 + (1 if world > 1 and args.exchange != "nccl" else 0)
+                                     + (1 if variant in (4, 7) and (world == 1 or args.exchange == "nccl") else 0)
                                      + (1 if world > 1 and args.exchange == "fused" else 0)),
             "roofline": {"bound": "tensor", "kernel": kernel, "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp8_peak, "traffic": traffic,

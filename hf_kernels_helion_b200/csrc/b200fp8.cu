@@ -454,8 +454,21 @@ int pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   return t_sk < t_pair ? B200FP8_VARIANT_PAIR256_SPLIT_SK : B200FP8_VARIANT_PAIR256_SPLIT;
 }
 
+// Whether the GEMM kernel reads the token scales (and, with up to 16 rows, A) where they are instead of copies that a
+// prep launch lays out for it: one launch less, 1.0-1.5 us a call, 3 us with up to 16 rows. Rows of As whose length and
+// address let a group of K blocks (two for 128-wide tiles, four otherwise) be loaded at once always do (4096 x 4096 x
+// 8192 133.3 -> 130.6 us, 256 x 28672 x 8192 79.0 -> 76.7, 37 x 28672 x 8192 43.4 -> 42.3, 4 x 2560 x 2048 8.2 -> 6.3);
+// one load of 32 sectors per K block keeps that gain up to about 64 K blocks per SM (345 x 1664 x 7808 17.0 -> 16.0,
+// 918 x 9216 x 6272, 95 of them, 58.5 -> 59.4).
+bool direct_scales(int variant, int64_t M, int64_t N, int64_t K, const float* As, int64_t ld_as, int sm_count) {
+  const int64_t bn = variant == B200FP8_VARIANT_TILE128 ? 128 : 256;
+  const int64_t group = bn == 128 ? 2 : 4;
+  if (ld_as % group == 0 && reinterpret_cast<uintptr_t>(As) % (group * 4) == 0) return true;
+  return ((M + 127) / 128) * ((N + bn - 1) / bn) * ((K + 127) / 128) <= 64 * static_cast<int64_t>(sm_count);
+}
+
 template <int BN>
-int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda, int64_t ldb, int sm_count,
+int launch_tile(const void* A, const void* B, GemmArgs args, int64_t lda, int64_t ldb, int sm_count,
                 cudaStream_t stream, int64_t sk_grid = 0, int cluster = 1) {
   CUtensorMap ta, tb;
   // Weight-streaming shapes: kernel forms with 16- or 64-row A slots and six or five pipeline stages
@@ -465,7 +478,11 @@ int launch_tile(const void* A, const void* B, const GemmArgs& args, int64_t lda,
   const bool decode = BN == 256 && args.M <= 64 && args.sk_split < 2 && args.n_dst == 1 && !args.mc_store &&
                       args.BsT == nullptr;
   const uint32_t a_rows = !decode ? 128u : args.M <= 16 ? 16u : 64u;
-  int st = make_tmap_u8(&ta, A, (args.a_from_prep && args.M < 16) ? 16 : args.M, args.K, lda, a_rows);
+  // (no copy of A: a box of the rows that exist; the slot's other rows keep what they held and give accumulator rows
+  // that are never stored)
+  const uint32_t box_rows = args.direct && args.M < static_cast<int64_t>(a_rows) ? static_cast<uint32_t>(args.M) : a_rows;
+  args.a_box_bytes = static_cast<int>(box_rows) * 128;
+  int st = make_tmap_u8(&ta, A, (args.a_from_prep && args.M < 16) ? 16 : args.M, args.K, lda, box_rows);
   if (st != B200FP8_OK) return st;
   st = make_tmap_u8(&tb, B, args.N, args.K, ldb, BN);
   if (st != B200FP8_OK) return st;
@@ -879,7 +896,10 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     fill_dst(args);
     // the copy of A the prep kernel writes: the quantised activations (b200fp8_linear), or A
     // copied (and zero-padded) to 16 rows when M <= 16
-    uint8_t* a_pad = (fused_q || M <= 16) ? static_cast<uint8_t*>(workspace) + tile_ast_bytes(M, K) : nullptr;
+    const bool direct = !fused_q && !fq.rowb && !multi && direct_scales(variant, M, N, K, As, ld_as, dev->sm_count);
+    args.direct = direct ? 1 : 0;
+    args.a_box_bytes = 0;
+    uint8_t* a_pad = (fused_q || (M <= 16 && !direct)) ? static_cast<uint8_t*>(workspace) + tile_ast_bytes(M, K) : nullptr;
     args.a_from_prep = a_pad != nullptr;
     args.sk_full = sk ? skp.full : 0;
     args.sk_split = sk ? skp.split : 0;
@@ -895,7 +915,7 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
           static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks));
       st = launch_status();
       if (st != B200FP8_OK) return st;
-    } else {
+    } else if (!direct) {
       const dim3 grid(static_cast<unsigned>(args.m_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
       tile_prep_kernel<<<dim3(grid.x, grid.y, a_pad != nullptr ? 2u : 1u), 256, 0, stream>>>(
           As, static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks), ld_as,

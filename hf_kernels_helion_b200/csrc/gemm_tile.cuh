@@ -54,6 +54,10 @@ struct GemmArgs {
   // mc_store = 1: dst[0] is a multimem address of a buffer replicated on every GPU of a multicast
   // group; the multi-destination kernel then re-reads each staged box row-wise and writes it
   // with multimem.st, once, and the NVSwitch delivers it to all GPUs (this one included).
+  // 1: no prep launch; the promotion warps read the token scales from As itself (row-major) and every warp that reads
+  // global memory first waits for the kernel before it in the stream (launched with programmatic serialisation)
+  int direct;
+  int a_box_bytes;   // single-CTA kernels: bytes of A per stage (box rows x 128)
   int a_from_prep;   // 1: A was re-laid by tile_prep_kernel (M <= 16: 16-row copy), the producer must wait for it
   int n_dst;
   int staged_store;
@@ -464,6 +468,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
         if (a_pending || ROWB) asm volatile("griddepcontrol.wait;" ::: "memory");
         a_pending = false;
       }
+      if (!ROWB && args.direct) asm volatile("griddepcontrol.wait;" ::: "memory");
       uint32_t tile_no = 0;   // ROWB: scale tables (pairs: chunks) loaded so far
       (void)tile_no;
       uint32_t pend_from = 0;
@@ -525,7 +530,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
             }
             continue;
           }
-          mbar_arrive_expect_tx(&full[s], Cfg::STAGE_BYTES);
+          mbar_arrive_expect_tx(&full[s], Cfg::B_BYTES + static_cast<uint32_t>(args.a_box_bytes));
           // one M block: the weight is read exactly once, the few activation rows by every CTA
           const bool hinted = A_ROWS < 128 || num_m == 1;
           auto load_a = [&](uint32_t stage, int kb_a, int m0_a) {
@@ -701,7 +706,11 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       // 128-byte load per warp and K block (row-major As would be 32 separate sectors)
       // (pair tiles of an odd last row block reach beyond the padded rows: those lanes read the last padded one, and
       // nothing of theirs is stored)
-      const float* as_col = args.AsT + (row < args.m_pad ? row : args.m_pad - 1);
+      // direct: row-major, read where it is, a group of K blocks of the lane's row in one load where it is aligned
+      const bool direct = !ROWB && args.direct;
+      const float* as_col = direct ? args.As + (row < M ? row : M - 1) * args.ld_as
+                                        : args.AsT + (row < args.m_pad ? row : args.m_pad - 1);
+      const int64_t as_step = direct ? 1 : args.m_pad;
       const float* bs_row = args.Bs + static_cast<int64_t>(nb) * args.ld_bs;
 
       // accumulators as 32-column groups of pairs: acc[g][j] = columns 32 g + 2 j, + 1
@@ -845,18 +854,38 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       constexpr int PF = (CHUNKS == 2 || ROWB) ? 2 : 4;
       float sa_c[PF], sb_c[PF], sa_n[PF], sb_n[PF];
       const int kb_last = seg.kb_end - 1;
+      const bool as_vec = direct && (args.ld_as % PF) == 0 &&
+                          (reinterpret_cast<uintptr_t>(args.As + seg.kb_begin) % (PF * 4)) == 0;
+      auto load_as = [&](int kb, float (&sa)[PF]) {
+        if (as_vec && kb + PF <= seg.kb_end) {
+          if constexpr (PF == 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(as_col + kb));
+            sa[0] = v.x;
+            sa[1] = v.y;
+            sa[PF - 2] = v.z;
+            sa[PF - 1] = v.w;
+          } else {
+            const float2 v = __ldg(reinterpret_cast<const float2*>(as_col + kb));
+            sa[0] = v.x;
+            sa[1] = v.y;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < PF; ++j) sa[j] = __ldg(as_col + (kb + j < seg.kb_end ? kb + j : kb_last) * as_step);
+        }
+      };
+      load_as(seg.kb_begin, sa_c);
 #pragma unroll
       for (int j = 0; j < PF; ++j) {
         const int k = seg.kb_begin + j < seg.kb_end ? seg.kb_begin + j : kb_last;
-        sa_c[j] = __ldg(as_col + k * args.m_pad);
         sb_c[j] = ROWB ? 1.f : __ldg(bs_row + k);
       }
       for (int kb0 = seg.kb_begin; ok && kb0 < seg.kb_end; kb0 += PF) {
+        load_as(kb0 + PF, sa_n);
 #pragma unroll
         for (int j = 0; j < PF; ++j) {
           int k = kb0 + PF + j;
           k = k < seg.kb_end ? k : kb_last;
-          sa_n[j] = __ldg(as_col + k * args.m_pad);
           sb_n[j] = ROWB ? 1.f : __ldg(bs_row + k);
         }
 #pragma unroll
