@@ -239,6 +239,24 @@ int make_tmap_u8(CUtensorMap* map, const void* base, int64_t rows, int64_t cols,
   return make_tmap(map, base, rows, cols, ld, box_rows, 0);
 }
 
+// Launch with programmatic stream serialisation: the kernel may be put on the device while the one before it in the
+// stream drains, and waits for it (pdl_wait) before it touches memory. Hides the launch latency between consecutive
+// kernels of a stream: 4096 x 8192 activations 18.4 -> 15.7 us call after call, a row-scaled 512 x 512 x 2048 product (two
+// prep launches) 20.5 -> 17.6. (The weight quantiser, one launch of many blocks, gained nothing.)
+template <typename... P, typename... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (a refusal is what launch_status reports)
+}
+
 int launch_status() { return cudaGetLastError() == cudaSuccess ? B200FP8_OK : B200FP8_ERR_LAUNCH; }
 
 // Scratch of b200fp8_gemm_decode_static: lives in the module image of every device that
@@ -667,11 +685,11 @@ int b200fp8_quant_act(const void* x, void* q, float* s, int64_t M, int64_t K, in
     // one unbroken run of 128-element groups: no row / column arithmetic in the kernel
     const unsigned blocks = static_cast<unsigned>((groups + 63) / 64);
     if ((reinterpret_cast<uintptr_t>(x) & 31u) == 0)
-      quant_act_contig_kernel<true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-          static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
+      launch_pdl(quant_act_contig_kernel<true>, dim3(blocks), static_cast<cudaStream_t>(stream),
+                 static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
     else
-      quant_act_contig_kernel<false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-          static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
+      launch_pdl(quant_act_contig_kernel<false>, dim3(blocks), static_cast<cudaStream_t>(stream),
+                 static_cast<const uint4*>(x), static_cast<uint4*>(q), s, groups);
     return launch_status();
   }
   const int64_t blocks_needed = (groups * 8 + 255) / 256;
@@ -679,11 +697,11 @@ int b200fp8_quant_act(const void* x, void* q, float* s, int64_t M, int64_t K, in
   const int grid = static_cast<int>(blocks_needed < max_blocks ? blocks_needed : max_blocks);
   // (the last pass of the loop steps at most one grid beyond the padded count)
   if (groups + 4 + static_cast<int64_t>(grid) * 32 <= 0xFFFFFFFFll)
-    quant_act_kernel<uint32_t><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
+    launch_pdl(quant_act_kernel<uint32_t>, dim3(grid), static_cast<cudaStream_t>(stream),
+               static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
   else
-    quant_act_kernel<int64_t><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
+    launch_pdl(quant_act_kernel<int64_t>, dim3(grid), static_cast<cudaStream_t>(stream),
+               static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), s, M, K, ldx, ldq, lds);
   return launch_status();
 }
 
@@ -910,16 +928,16 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     if (fused_q) {
       const int64_t rows_q = M < 16 ? 16 : M;
       const int64_t threads = args.m_pad * kblocks * 8;
-      tile_prep_quant_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-          static_cast<const __nv_bfloat16*>(fq.x_bf16), fq.ldx, a_pad, align_up(K, 16), rows_q,
-          static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks));
+      launch_pdl(tile_prep_quant_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), stream,
+                 static_cast<const __nv_bfloat16*>(fq.x_bf16), fq.ldx, a_pad, align_up(K, 16), rows_q,
+                 static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks));
       st = launch_status();
       if (st != B200FP8_OK) return st;
     } else if (!direct) {
       const dim3 grid(static_cast<unsigned>(args.m_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
-      tile_prep_kernel<<<dim3(grid.x, grid.y, a_pad != nullptr ? 2u : 1u), 256, 0, stream>>>(
-          As, static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks), ld_as,
-          static_cast<const uint8_t*>(A), a_pad, K, lda, align_up(K, 16));
+      launch_pdl(tile_prep_kernel, dim3(grid.x, grid.y, a_pad != nullptr ? 2u : 1u), stream, As,
+                 static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks), ld_as,
+                 static_cast<const uint8_t*>(A), a_pad, K, lda, align_up(K, 16));
       st = launch_status();
       if (st != B200FP8_OK) return st;
     }
@@ -930,8 +948,8 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       // second transposition: the row scales of B, K-block-major (same kernel, B in the role of A)
       float* bst = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix + (sk ? skp.partial_bytes : 0));
       const dim3 grid(static_cast<unsigned>(args.n_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
-      tile_prep_kernel<<<grid, 256, 0, stream>>>(Bs, bst, N, args.n_pad, static_cast<int>(kblocks), ld_bs, nullptr,
-                                                 nullptr, K, 0, 0);
+      launch_pdl(tile_prep_kernel, grid, stream, Bs, bst, N, args.n_pad, static_cast<int>(kblocks), ld_bs, nullptr, nullptr,
+                 K, 0, 0);
       st = launch_status();
       if (st != B200FP8_OK) return st;
       args.BsT = bst;

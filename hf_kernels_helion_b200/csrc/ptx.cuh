@@ -32,6 +32,11 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch. wait: until the kernel before this one in the stream has ended and its writes are
+// visible (returns at once in a kernel launched without the attribute); trigger: the next kernel may be launched.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------- CTA pairs (clusters of two)
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {

@@ -11,6 +11,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace b200fp8 {
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -144,6 +146,8 @@ template <bool WIDE>
 __global__ void __launch_bounds__(256)
 quant_act_contig_kernel(const uint4* __restrict__ x, uint4* __restrict__ q, float* __restrict__ s,
                         int64_t total_groups) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   const int64_t g = t >> 2;
   const int sub = threadIdx.x & 3;
@@ -176,6 +180,8 @@ template <typename Idx>
 __global__ void __launch_bounds__(256)
 quant_act_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ s, int64_t M,
                  int64_t K, int64_t ldx, int64_t ldq, int64_t lds) {
+  pdl_wait();
+  pdl_trigger();
   const Idx groups_per_row = static_cast<Idx>((K + 127) / 128);
   const Idx total_groups = static_cast<Idx>(M) * groups_per_row;
   const int sub = threadIdx.x & 7;
