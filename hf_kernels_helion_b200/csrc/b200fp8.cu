@@ -407,12 +407,20 @@ Pick pick_form(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   // K = 8192: the plain 128x256 tile kernel (46 us at M = 16, 5.1 TB/s with 112 of 148 SMs busy)
   // beats the swap-AB stream-K kernel (65 us), so AUTO does not pick that one.
   // (two row blocks, M in 129..256, go to the CTA pairs below when the device runs them: 79.5 vs 84-86 us at M = 256)
-  if (M <= 128 || (M <= 256 && (N <= 128 || !pair_ok))) {
-    const int64_t bn = N > 128 ? 256 : 128;
-    return {N > 128 ? B200FP8_VARIANT_TILE256 : B200FP8_VARIANT_TILE128,
-            6.0 + 0.43 * kb * waves(num_m * ((N + bn - 1) / bn), sm_count)};
+  // One row block: 128-wide tiles as long as each has an SM to itself - more SMs pull on the weight, and four accumulator
+  // stages instead of two are in flight (29 x 13952 x 1680 9.2 vs 11.9 us, 50 x 1024 x 464 4.8 vs 6.9, 1 x 8704 x 544 5.2 vs
+  // 6.2) - and 256-wide ones beyond (3 x 21376 x 7808, 167 narrow tiles: 58.0 vs 32.6).
+  if (M <= 128) {
+    const int64_t narrow = (N + 127) / 128;
+    if (narrow <= sm_count) return {B200FP8_VARIANT_TILE128, 4.5 + 0.30 * kb};
+    return {B200FP8_VARIANT_TILE256, 6.0 + 0.43 * kb * waves((N + 255) / 256, sm_count)};
   }
-  Pick best = {B200FP8_VARIANT_TILE128, 6.0 + waves(num_m * ((N + 127) / 128), sm_count) * (0.405 * kb + 0.5)};
+  if (M <= 256 && (N <= 128 || !pair_ok))
+    return {N > 128 ? B200FP8_VARIANT_TILE256 : B200FP8_VARIANT_TILE128, 6.0 + 0.43 * kb};
+  // (128 x 128 tiles: 0.31 us per K block on a few SMs, 0.385 when all of them load operands from L2)
+  const int64_t tiles = num_m * ((N + 127) / 128);
+  const double share = 0.385 * static_cast<double>(tiles < sm_count ? tiles : sm_count) / sm_count;
+  Pick best = {B200FP8_VARIANT_TILE128, 5.5 + waves(tiles, sm_count) * ((share > 0.31 ? share : 0.31) * kb + 0.5)};
   auto consider = [&best](int variant, double us) {
     if (us < best.us) best = {variant, us};
   };
@@ -433,7 +441,7 @@ int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
 
 // CTAs per tile (2..8) for products whose 128 x 128 tiles leave SMs idle: the K blocks of a tile are cut over a cluster
 // (gemm_cluster_kernel), as far as all clusters are resident at once. 1: another form is estimated to be faster.
-// Cutting costs about 2 us (two cluster barriers and the addition through distributed shared memory), so that products of
+// Cutting costs 1-2 us (two cluster barriers and the addition through distributed shared memory), so that products of
 // fewer than 12 K blocks stay whole. Measured, one / two / four CTAs per tile, us: 4 x 2560 x 2048 12.9 / 9.0 / 8.1,
 // 64 x 2048 x 4096 20.1 / 12.3 / 9.4, 512 x 512 x 2048 11.4 / 11.3 / 9.2, 512 x 512 x 8192 28.9 / 19.5 / 13.3,
 // 1 x 8192 x 8192 34.0 / 17.6 / - (more clusters than fit: 22.3).
@@ -444,7 +452,7 @@ int cluster_split(int64_t M, int64_t N, int64_t K, const int* clusters, double o
   if (kblocks < 12) return best;
   for (int c = 2; c <= kClusterMax; ++c) {
     if (tiles > clusters[c] || kblocks < 2 * c) continue;
-    const double us = 8.2 + 0.405 * static_cast<double>((kblocks + c - 1) / c);
+    const double us = (M <= 128 ? 5.3 : 7.5) + 0.33 * static_cast<double>((kblocks + c - 1) / c);
     if (us < other_us) {
       other_us = us;
       best = c;
