@@ -933,6 +933,9 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     args.partial = sk ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix) : nullptr;
     args.AsT = static_cast<const float*>(workspace);
     args.m_pad = align_up(M, 128);
+    args.n_pad = align_up(N, 128);
+    args.BsT = nullptr;
+    args.rowb_table = 0;
     if (fused_q) {
       const int64_t rows_q = M < 16 ? 16 : M;
       const int64_t threads = args.m_pad * kblocks * 8;
@@ -942,26 +945,22 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       st = launch_status();
       if (st != B200FP8_OK) return st;
     } else if (!direct) {
-      const dim3 grid(static_cast<unsigned>(args.m_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
-      launch_pdl(tile_prep_kernel, dim3(grid.x, grid.y, a_pad != nullptr ? 2u : 1u), stream, As,
-                 static_cast<float*>(workspace), M, args.m_pad, static_cast<int>(kblocks), ld_as,
-                 static_cast<const uint8_t*>(A), a_pad, K, lda, align_up(K, 16));
+      const ScaleCopy token = {As, static_cast<float*>(workspace), M, args.m_pad, ld_as};
+      ScaleCopy weight = {nullptr, nullptr, 0, 0, 0};
+      if (fq.rowb) {
+        // the row scales of B, K-block-major, behind the token scales, the copy of A and the partial tiles
+        args.BsT = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix + (sk ? skp.partial_bytes : 0));
+        args.rowb_table = kblocks <= kRowbTableKb ? 1 : 0;
+        weight = {Bs, const_cast<float*>(args.BsT), N, args.n_pad, ld_bs};
+      }
+      const int64_t rows = weight.pad > token.pad ? weight.pad : token.pad;
+      launch_pdl(tile_prep_kernel,
+                 dim3(static_cast<unsigned>(rows / 32), static_cast<unsigned>((kblocks + 31) / 32),
+                      a_pad != nullptr ? 3u : fq.rowb ? 2u : 1u),
+                 stream, token, weight, static_cast<int>(kblocks), static_cast<const uint8_t*>(A), a_pad, M, K, lda,
+                 align_up(K, 16));
       st = launch_status();
       if (st != B200FP8_OK) return st;
-    }
-    args.BsT = nullptr;
-    args.rowb_table = 0;
-    args.n_pad = align_up(N, 128);
-    if (fq.rowb) {
-      // second transposition: the row scales of B, K-block-major (same kernel, B in the role of A)
-      float* bst = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + prefix + (sk ? skp.partial_bytes : 0));
-      const dim3 grid(static_cast<unsigned>(args.n_pad / 32), static_cast<unsigned>((kblocks + 31) / 32));
-      launch_pdl(tile_prep_kernel, grid, stream, Bs, bst, N, args.n_pad, static_cast<int>(kblocks), ld_bs, nullptr, nullptr,
-                 K, 0, 0);
-      st = launch_status();
-      if (st != B200FP8_OK) return st;
-      args.BsT = bst;
-      args.rowb_table = kblocks <= kRowbTableKb ? 1 : 0;
     }
     args.As = As;
     args.Bs = Bs;

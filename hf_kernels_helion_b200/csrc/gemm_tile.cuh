@@ -1343,21 +1343,29 @@ peer_barrier_kernel(PeerFlags flags, int n, int rank, uint32_t epoch, long long 
   }
 }
 
-// Launch-side preparation of one GEMM call, grid = (m_pad / 32, ceil(num_kb / 32), 1 or 2):
-//   z = 0  AsT[kb][m] = As[m][kb] for m < M, 0 for M <= m < m_pad: 32 x 32 tiles through
-//          shared memory so that both the row-major reads and the K-block-major writes are
-//          coalesced;
-//   z = 1  (only when M <= 16) A_pad[16][lda_pad] = A with zero rows appended: TMA boxes over a
-//          tensor of fewer than 16 rows measured ~20 % slower on B200 than over 16 rows.
+// One K-block-major copy of row-major scales, src [rows, num_kb] -> dst [num_kb][pad], zero for rows <= r < pad.
+struct ScaleCopy {
+  const float* src;
+  float* dst;
+  int64_t rows, pad, ld;
+};
+
+// Launch-side preparation of one GEMM call, grid = (32-row blocks of the longer scale matrix, ceil(num_kb / 32), pieces).
+// Piece blockIdx.z = 0 is the first scale copy, 1 the second (row-scaled B: both in one launch; a launch of its own for the
+// second cost 2-3 us a call), 2 the copy of A:
+//   scales  32 x 32 tiles through shared memory so that both the row-major reads and the K-block-major writes are
+//           coalesced;
+//   A       (only when M <= 16) A_pad[16][lda_pad] = A with zero rows appended: TMA boxes over a
+//           tensor of fewer than 16 rows measured ~20 % slower on B200 than over 16 rows.
 __global__ void __launch_bounds__(256)
-tile_prep_kernel(const float* __restrict__ As, float* __restrict__ AsT, int64_t M, int64_t m_pad, int num_kb,
-                 int64_t ld_as, const uint8_t* __restrict__ A, uint8_t* __restrict__ A_pad, int64_t K, int64_t lda,
-                 int64_t lda_pad) {
+tile_prep_kernel(const ScaleCopy first, const ScaleCopy second, int num_kb, const uint8_t* __restrict__ A,
+                 uint8_t* __restrict__ A_pad, int64_t M, int64_t K, int64_t lda, int64_t lda_pad) {
   // let the GEMM kernel that follows (launched with programmatic stream serialisation) start its prologue and its weight
   // loads once the kernel before this one is done; the warps that read what this grid writes wait for it
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.z == 1) {
+  if (blockIdx.z == 2) {
+    if (A_pad == nullptr) return;
     const int64_t chunks_per_row = lda_pad / 16;
     const int64_t total = 16 * chunks_per_row;
     const int64_t nthreads = static_cast<int64_t>(gridDim.x) * gridDim.y * blockDim.x;
@@ -1379,22 +1387,24 @@ tile_prep_kernel(const float* __restrict__ As, float* __restrict__ AsT, int64_t 
     }
     return;
   }
+  const ScaleCopy& s = blockIdx.z == 0 ? first : second;
   __shared__ float t[32][33];
   const int64_t m0 = static_cast<int64_t>(blockIdx.x) * 32;
+  if (s.dst == nullptr || m0 >= s.pad) return;
   const int kb0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
 #pragma unroll
   for (int i = 0; i < 32; i += 8) {
     const int64_t m = m0 + ty + i;
     const int kb = kb0 + tx;
-    t[ty + i][tx] = (m < M && kb < num_kb) ? __ldg(As + m * ld_as + kb) : 0.f;
+    t[ty + i][tx] = (m < s.rows && kb < num_kb) ? __ldg(s.src + m * s.ld + kb) : 0.f;
   }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 32; i += 8) {
     const int kb = kb0 + ty + i;
     const int64_t m = m0 + tx;
-    if (kb < num_kb && m < m_pad) AsT[static_cast<int64_t>(kb) * m_pad + m] = t[tx][ty + i];
+    if (kb < num_kb && m < s.pad) s.dst[static_cast<int64_t>(kb) * s.pad + m] = t[tx][ty + i];
   }
 }
 
