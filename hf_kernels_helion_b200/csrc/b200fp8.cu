@@ -514,8 +514,8 @@ int launch_tile(const void* A, const void* B, GemmArgs args, int64_t lda, int64_
   if (st != B200FP8_OK) return st;
   const int64_t tiles = ((args.M + 127) / 128) * ((args.N + BN - 1) / BN);
   const int grid = sk_grid > 0 ? static_cast<int>(sk_grid) : static_cast<int>(tiles < sm_count ? tiles : sm_count);
-  // Programmatic dependent launch: the kernel may begin (barrier set-up, TMEM allocation,
-  // operand loads) while the tile_prep_kernel enqueued just before it is still running.
+  // Programmatic dependent launch: the kernel may begin (barrier set-up, TMEM allocation, and behind a prep
+  // launch of the same call also operand loads) while the kernel enqueued just before it is still running.
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -18,7 +18,8 @@
 // Forms of the same body (template parameters of gemm_tile_body): 128- or 256-wide tiles; a
 // multi-destination epilogue (TMA stores or multimem stores of every finished box into several
 // [M, N] buffers: the N-sharded multi-GPU exchange); tail split-K; row-scaled B; decode forms
-// with 16- or 64-row A slots; and CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair).
+// with 16- or 64-row A slots; clusters whose CTAs share one tile along K; and CTA pairs (tcgen05
+// cta_group::2, 256 x 256 tiles per pair).
 #pragma once
 
 #include <cuda_bf16.h>

@@ -120,7 +120,7 @@ int b200fp8_quant_weight(const void* w, void* q, float* s,
  * M, N, K otherwise arbitrary (ragged edges are masked). M == 0 or N == 0 is a
  * no-op; K == 0 writes zeros.
  *
- * `workspace` holds per-call scratch (a K-block-major copy of As for every variant, plus
+ * `workspace` holds per-call scratch (room for a K-block-major copy of As for every variant, plus
  * the fp32 partial tiles of B200FP8_VARIANT_STREAMK); size it with
  * b200fp8_gemm_workspace_bytes for the same (M, N, K, variant), align it to 256 bytes. Its
  * contents need no initialisation.
