@@ -66,6 +66,9 @@ int device_info(const DeviceInfo** out) {
       opt_in(reinterpret_cast<const void*>(&gemm_tile_kernel<128, 0>), TileCfg<128, false>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_kernel<256, 0>), TileCfg<256, false>::SMEM_BYTES);
       opt_in(reinterpret_cast<const void*>(&gemm_cluster_kernel), TileCfg<128, false>::SMEM_BYTES);
+      opt_in(reinterpret_cast<const void*>(&gemm_cluster_rowb_kernel), TileCfg<128, false, 128, 0, true>::SMEM_BYTES);
+      regs_ok(reinterpret_cast<const void*>(&gemm_cluster_rowb_kernel), TileCfg<128>::THREADS,
+              128 * TileCfg<128>::REGS_CONTROL + 256 * TileCfg<128>::REGS_EPILOGUE);
       regs_ok(reinterpret_cast<const void*>(&gemm_cluster_kernel), TileCfg<128>::THREADS,
               128 * TileCfg<128>::REGS_CONTROL + 256 * TileCfg<128>::REGS_EPILOGUE);
       opt_in(reinterpret_cast<const void*>(&gemm_tile_multi_kernel<128>), TileCfg<128, true>::SMEM_BYTES);
@@ -445,14 +448,17 @@ int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
 // fewer than 12 K blocks stay whole. Measured, one / two / four CTAs per tile, us: 4 x 2560 x 2048 12.9 / 9.0 / 8.1,
 // 64 x 2048 x 4096 20.1 / 12.3 / 9.4, 512 x 512 x 2048 11.4 / 11.3 / 9.2, 512 x 512 x 8192 28.9 / 19.5 / 13.3,
 // 1 x 8192 x 8192 34.0 / 17.6 / - (more clusters than fit: 22.3).
-int cluster_split(int64_t M, int64_t N, int64_t K, const int* clusters, double other_us) {
+// With row-scaled B a K block takes longer and cutting pays more: 512 x 512 x 2048 16.0 -> 11.5 us, 38 x 1024 x 4096 21.7 -> 9.6,
+// 2 x 512 x 8192 39.2 -> 12.0, 256 x 2048 x 4096 (split tail of pair tiles before) 19.9 -> 14.5.
+int cluster_split(int64_t M, int64_t N, int64_t K, const int* clusters, double other_us, bool rowb) {
   const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
   const int64_t kblocks = (K + 127) / 128;
   int best = 1;
   if (kblocks < 12) return best;
   for (int c = 2; c <= kClusterMax; ++c) {
     if (tiles > clusters[c] || kblocks < 2 * c) continue;
-    const double us = (M <= 128 ? 5.3 : 7.5) + 0.33 * static_cast<double>((kblocks + c - 1) / c);
+    const double kb = static_cast<double>((kblocks + c - 1) / c);
+    const double us = rowb ? 10.0 + 0.56 * kb : (M <= 128 ? 5.3 : 7.5) + 0.33 * kb;
     if (us < other_us) {
       other_us = us;
       best = c;
@@ -467,17 +473,18 @@ int cluster_split(int64_t M, int64_t N, int64_t K, const int* clusters, double o
 // prologue, the fix-up pass of the split tail takes 5. Measured, 128 x 128 / pair / pair with split tail, us:
 // 4096 x 4096 x 8192 268.6 / 241.8 / 221.8, 2048 x 2048 x 4096 46.8 / 36.9 / 36.8, 256 x 4096 x 4096 25.2 / 35.1 / 20.5,
 // 512 x 2048 x 2048 16.7 / 22.0 / 17.6, 8192 x 4096 x 7168 469.8 / 386.4 / 395.5.
-int pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
-  if (pairs < 1 || M <= 128) return B200FP8_VARIANT_TILE128;
+Pick pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
   const double kb = static_cast<double>((K + 127) / 128);
   const double t128 = 0.56 * kb * static_cast<double>((tiles + sm_count - 1) / sm_count);
+  if (pairs < 1 || M <= 128) return {B200FP8_VARIANT_TILE128, 8.0 + t128};
   const TileSkPlan p = pair_sk_plan(M, N, K, pairs);
   const double full = 0.87 * kb * static_cast<double>(p.full / pairs);
   const double t_pair = full + (p.tail > 0 ? 0.87 * kb : 0.0);
   const double t_sk = p.split >= 2 ? full + 0.87 * p.kb_per + 5.0 : t_pair;
-  if (t128 <= t_pair && t128 <= t_sk) return B200FP8_VARIANT_TILE128;
-  return t_sk < t_pair ? B200FP8_VARIANT_PAIR256_SPLIT_SK : B200FP8_VARIANT_PAIR256_SPLIT;
+  if (t128 <= t_pair && t128 <= t_sk) return {B200FP8_VARIANT_TILE128, 8.0 + t128};
+  if (t_sk < t_pair) return {B200FP8_VARIANT_PAIR256_SPLIT_SK, 8.0 + t_sk};
+  return {B200FP8_VARIANT_PAIR256_SPLIT, 8.0 + t_pair};
 }
 
 // Whether the GEMM kernel reads the token scales (and, with up to 16 rows, A) where they are instead of copies that a
@@ -530,7 +537,7 @@ int launch_tile(const void* A, const void* B, GemmArgs args, int64_t lda, int64_
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t err;
-  if (BN == 128 && cluster > 1) {
+  if (BN == 128 && cluster > 1 && args.BsT == nullptr) {
     cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
     cfg.numAttrs = 2;
     cfg.dynamicSmemBytes = TileCfg<128, false>::SMEM_BYTES;
@@ -553,7 +560,13 @@ int launch_tile(const void* A, const void* B, GemmArgs args, int64_t lda, int64_
                    static_cast<uint32_t>(kblocks < kRowbTableKb ? kblocks : kRowbTableKb), 1);
     if (st != B200FP8_OK) return st;
     cfg.dynamicSmemBytes = TileCfg<128, false, 128, 0, true>::SMEM_BYTES;
-    err = cudaLaunchKernelEx(&cfg, gemm_tile_rowb_kernel<128>, ta, tb, tbst, args);
+    if (cluster > 1) {
+      cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
+      cfg.numAttrs = 2;
+      err = cudaLaunchKernelEx(&cfg, gemm_cluster_rowb_kernel, ta, tb, tbst, args);
+    } else {
+      err = cudaLaunchKernelEx(&cfg, gemm_tile_rowb_kernel<128>, ta, tb, tbst, args);
+    }
   } else if (args.mc_store) {
     cfg.dynamicSmemBytes = TileCfg<BN, true>::SMEM_BYTES;
     err = cudaLaunchKernelEx(&cfg, gemm_tile_mc_kernel<BN>, ta, tb, args);
@@ -874,7 +887,9 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     auto_us = p.us;
   }
   if (fq.rowb) {
-    variant = pick_rowb(M, N, K, dev->sm_count, staged ? dev->pair_clusters : 0);
+    const Pick p = pick_rowb(M, N, K, dev->sm_count, staged ? dev->pair_clusters : 0);
+    variant = p.variant;
+    auto_us = p.us;
     // (a workspace without room for the partial tiles: the same tiles without the split tail)
     if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK &&
         static_cast<int64_t>(workspace_bytes) < tile_workspace_bytes(M, K) + bst_bytes(N, K) +
@@ -882,7 +897,8 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       variant = B200FP8_VARIANT_PAIR256_SPLIT;
   }
   const bool multi = n_dst > 1 || mc;
-  const int cluster = auto_variant && !multi && !fq.rowb ? cluster_split(M, N, K, dev->clusters, auto_us) : 1;
+  const int cluster =
+      (auto_variant || fq.rowb) && !multi ? cluster_split(M, N, K, dev->clusters, auto_us, fq.rowb) : 1;
   if (cluster > 1) variant = B200FP8_VARIANT_TILE128;
   if (fq.rowb && (multi || fused_q)) return B200FP8_ERR_VARIANT;
   // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room
@@ -1072,7 +1088,7 @@ int64_t b200fp8_gemm_rowscale_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M < 0 || N < 0 || K < 0) return -static_cast<int64_t>(B200FP8_ERR_SHAPE);
   if (M == 0 || N == 0 || K == 0) return 0;
   const int pairs = b200fp8_gemm_pair_clusters();
-  const bool sk = pick_rowb(M, N, K, sm_count_or_default(), pairs) == B200FP8_VARIANT_PAIR256_SPLIT_SK;
+  const bool sk = pick_rowb(M, N, K, sm_count_or_default(), pairs).variant == B200FP8_VARIANT_PAIR256_SPLIT_SK;
   return tile_workspace_bytes(M, K) + bst_bytes(N, K) + (sk ? pair_sk_plan(M, N, K, pairs).partial_bytes : 0);
 }
 

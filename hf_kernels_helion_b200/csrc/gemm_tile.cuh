@@ -371,7 +371,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
   constexpr uint32_t H = Cfg::HALVES;
   static_assert(!(PAIR && MC), "pair kernels: plain or TMA-store output");
   static_assert(!(PAIR == 1 && ROWB), "row-scaled B: the split pair form only");
-  static_assert(!CL || (!PAIR && !MULTI && !SK && !ROWB && BN == 128), "cluster split: plain 128-wide tiles");
+  static_assert(!CL || (!PAIR && !MULTI && !SK && BN == 128), "cluster split: plain 128-wide tiles");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1126,6 +1126,13 @@ __global__ void __launch_bounds__(TileCfg<128, false>::THREADS, 1)
 gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmArgs args) {
   gemm_tile_body<128, false, 0, false, false, 128, 0, true>(tmap_a, tmap_b, args, nullptr);
+}
+
+// The same with row-scaled B; every CTA holds the scales of the whole depth of its tile.
+__global__ void __launch_bounds__(TileCfg<128, false>::THREADS, 1)
+gemm_cluster_rowb_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                         const __grid_constant__ CUtensorMap tmap_bst, const GemmArgs args) {
+  gemm_tile_body<128, false, 0, false, true, 128, 0, true>(tmap_a, tmap_b, args, nullptr, &tmap_bst);
 }
 
 // CTA-pair forms (launch with cluster dimension 2 and an even grid): 256 x 256 tiles per pair.

@@ -98,3 +98,20 @@ def test_rowscale_on_cta_pairs(device, M, N, K):
     assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.float32), out32)
     assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.bfloat16), out32.to(torch.bfloat16))
     runtime.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1536), (4, 1408, 2064), (97, 201, 1664), (130, 384, 8192), (300, 264, 16400)])
+def test_rowscale_on_clusters(device, M, N, K):
+    """Few tiles: the CTAs of a cluster share one along K. Uneven ranges, a short last K block, ragged rows and columns, K up to
+    and beyond the shared-memory table of scales."""
+    A, B, As, Bs = oracle.make_rowscale_inputs(M, N, K, M + N + K)
+    d = [t.to(device) for t in (A, B, As, Bs)]
+    a = (d[0].double() * d[2].double().repeat_interleave(128, 1)[:, :K])
+    ref = a @ (d[1].double() * d[3].double().repeat_interleave(128, 1)[:, :K]).T
+    out32 = runtime.gemm_rowscale(*d, 128, torch.float32)
+    # fp32 accumulation over K blocks, exact fp32 products inside one: a few roundings of 2^-24 each per K block
+    rel = ((out32.double() - ref).norm() / ref.norm()).item()
+    assert rel <= 2.0 ** -24 * (2 + -(-K // 128)) ** 0.5 * 4
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.float32), out32)
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.bfloat16), out32.to(torch.bfloat16))
+    runtime.check_device_status()
