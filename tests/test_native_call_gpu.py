@@ -124,3 +124,60 @@ def test_graph_capture(device, operands):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+HOLD = r"""
+#include <time.h>
+volatile int entered, released;
+/* stands in for a library call that takes its time: at most one second, less if somebody sets `released` meanwhile */
+int hold(void) {
+  struct timespec ms = {0, 1000000};
+  int i;
+  entered = 1;
+  for (i = 0; i < 1000 && !released; ++i) nanosleep(&ms, 0);
+  return released ? 0 : 10;
+}
+"""
+
+
+def test_other_threads_run_while_a_call_is_in_the_library(device, operands, tmp_path):
+    """A launch can wait (a full queue, an allocation), and what it waits for may need another Python thread: the call gives
+    the interpreter up meanwhile, as the registered ops do."""
+    import ctypes
+    import subprocess
+    import time
+
+    from hf_kernels_helion_b200 import _lib
+
+    A, B, As, Bs = operands
+    (tmp_path / "hold.c").write_text(HOLD)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(tmp_path / "hold.so"), str(tmp_path / "hold.c")], check=True)
+    held = ctypes.CDLL(str(tmp_path / "hold.so"))
+    entered, released = (ctypes.c_int.in_dll(held, n) for n in ("entered", "released"))
+    x = torch.zeros(4, 512, device=device, dtype=torch.bfloat16)
+    calls = [lambda: _native(A, B, As, Bs), lambda: _native(A, B, As, Bs.repeat_interleave(128, 0), 128, torch.bfloat16),
+             lambda: runtime.native.linear(x, B, Bs, torch.bfloat16), lambda: runtime.native.act_quant(x, 128),
+             lambda: runtime.native.weight_quant(x, 128)]
+    hold = ctypes.cast(held.hold, ctypes.c_void_p).value
+    size = [ctypes.cast(getattr(_lib.load(), f"b200fp8_{n}_workspace_bytes"), ctypes.c_void_p).value
+            for n in ("gemm", "gemm_rowscale", "linear")]
+
+    def let_go():
+        while not entered.value and time.monotonic() < limit:
+            time.sleep(0.001)
+        released.value = 1
+
+    results = []
+    try:
+        runtime.native.bind(hold, size[0], hold, size[1], hold, size[2], hold, hold)
+        for call in calls:
+            entered.value = released.value = 0
+            limit = time.monotonic() + 5
+            other = threading.Thread(target=let_go)
+            other.start()
+            results.append(call() is not None)
+            other.join()
+    finally:
+        _lib.load_native()      # binds the library again
+    assert results == [True] * len(calls)
+    assert torch.equal(_native(*operands), runtime.gemm(A, B, As, Bs, 128, 128, torch.float32))
