@@ -6,6 +6,8 @@ returns a non-zero status, a RuntimeError is raised.
 from __future__ import annotations
 
 import ctypes
+import sys
+import warnings
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
@@ -76,14 +78,28 @@ def load():
     return _lib
 
 
+def native_tag() -> str:
+    """The torch and the Python of this process, as the native call module names those it was built for."""
+    import torch
+
+    return f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+
+
 def load_native():
-    """The module built from csrc/torch_call.cpp, bound to the library; raise if either has not been built."""
+    """The module built from csrc/torch_call.cpp, bound to the library. None, with a warning, where it has not been
+    built or was built for another torch or Python: every call then takes the way through the registered ops, which
+    launches the same kernels and needs only the library. Raises if the library itself is missing."""
     lib = load()
     try:
         from . import _torch_call
+        built_for = getattr(_torch_call, "built_for", "an unnamed torch and Python")
+        why = None if built_for == native_tag() else f"was built for {built_for}"
     except ImportError as e:
-        raise RuntimeError(f"{NATIVE_PATH} is missing or does not load ({e}): build it with "
-                           "`python -m hf_kernels_helion_b200.build`") from e
+        why = f"does not load ({e})"
+    if why is not None:
+        warnings.warn(f"{NATIVE_PATH} {why}; this is {native_tag()}. Calls go through the registered torch ops, at 30-50 us "
+                      "of host time each. Build it with `python -m hf_kernels_helion_b200.build`", RuntimeWarning, stacklevel=2)
+        return None
     _torch_call.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in (
         "b200fp8_gemm", "b200fp8_gemm_workspace_bytes", "b200fp8_gemm_rowscale", "b200fp8_gemm_rowscale_workspace_bytes",
         "b200fp8_linear", "b200fp8_linear_workspace_bytes", "b200fp8_quant_act", "b200fp8_quant_weight")))

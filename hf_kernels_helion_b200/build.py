@@ -14,6 +14,8 @@ import subprocess
 import sys
 from pathlib import Path
 
+from . import _lib
+
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libb200fp8.so"
@@ -40,8 +42,13 @@ def _is_stale(target: Path, sources) -> bool:
     return not target.exists() or any(p.stat().st_mtime > target.stat().st_mtime for p in sources)
 
 
+def _native_is_stale() -> bool:
+    """Older than its sources, or built for another torch or Python (it carries the names of its own as a string)."""
+    return _is_stale(NATIVE_PATH, NATIVE_SOURCES) or _lib.native_tag().encode() + b"\0" not in NATIVE_PATH.read_bytes()
+
+
 def is_stale() -> bool:
-    return _is_stale(LIB_PATH, SOURCES + HEADERS) or _is_stale(NATIVE_PATH, NATIVE_SOURCES)
+    return _is_stale(LIB_PATH, SOURCES + HEADERS) or _native_is_stale()
 
 
 def _native_command() -> list[str]:
@@ -53,7 +60,7 @@ def _native_command() -> list[str]:
     root = str(Path(find_nvcc()).resolve().parent.parent)
     includes = cpp_extension.include_paths() + [sysconfig.get_path("include"), os.path.join(root, "include")]
     cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DB200FP8_BUILT_FOR="{_lib.native_tag()}"']
     for d in includes:
         cmd += ["-isystem", d]
     cmd += [str(NATIVE_SOURCES[0]), "-o", str(NATIVE_PATH)]
@@ -76,7 +83,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if verbose:
             cmd += ["-Xptxas", "-v"]
         _run(cmd + ["-o", str(LIB_PATH), *map(str, SOURCES)], verbose)
-    if force or _is_stale(NATIVE_PATH, NATIVE_SOURCES):
+    if force or _native_is_stale():
         _run(_native_command(), verbose)
     return LIB_PATH
 

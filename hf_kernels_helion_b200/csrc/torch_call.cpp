@@ -1,13 +1,16 @@
 // The short way from a Python call to the C ABI (include/b200fp8.h): for ordinary eager CUDA tensors one
 // native function checks the operands, takes the result and the scratch from torch's caching allocator and
-// enqueues the launches, without the interpreter lock. What it does not know to be that case (another layout, a tensor subclass, a grad or
-// a dual tensor, tracing, an active torch mode or profiler, a bad argument) makes it return None, and the
-// Python path - registered torch op, argument errors, copies of unusual layouts - handles the call as it
-// would without this file. A call through the registered op and ctypes costs 30-50 us of host time, more
-// than the kernels of most decode and small-matrix calls take.
+// enqueues the launches, without the interpreter lock. What it does not know to be that case (another layout, a
+// tensor subclass, a grad or a dual tensor, tracing, an active torch mode or profiler, a bad argument) makes it
+// return None, and the Python path - registered torch op, argument errors, copies of unusual layouts - handles
+// the call as it would without this file. A call through the registered op and ctypes costs 30-50 us of host
+// time, more than the kernels of most decode and small-matrix calls take.
 //
 // Scratch belongs to one call: it comes from the caching allocator of the current stream, is given back when
 // the call returns (stream order keeps it safe) and is never shared between threads, streams or graphs.
+//
+// The file reads torch's and Python's own structures, so what it compiles to works with the torch and the Python it
+// was built for and no others: `built_for` names them, and _lib.load_native compares it before it calls anything here.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -24,6 +27,10 @@
 #include <cstdlib>
 
 #include "../../include/b200fp8.h"
+
+#ifndef B200FP8_BUILT_FOR
+#error "B200FP8_BUILT_FOR: a string that names the torch and the Python this is built for"
+#endif
 
 namespace {
 
@@ -339,4 +346,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_call", nullptr, -1, kMetho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_call(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__torch_call(void) {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", B200FP8_BUILT_FOR) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

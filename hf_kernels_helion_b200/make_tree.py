@@ -14,7 +14,9 @@ flat `__init__.py` by path) so that `PYTHONPATH=OUT_DIR/torch-cuda` makes
 
 `metadata.json` keeps the reference's name, id and backend and has an empty `python-depends`
 (the reference's is ["helion"], build.toml:9). The tree is binary: it carries the built
-`libb200fp8.so` and `_torch_call.so`, not the sources.
+`libb200fp8.so` and `_torch_call.so`, not the sources. `_torch_call.so` (the short way for eager calls) is used by the
+torch and the Python it was built with, those of the process that writes the tree; under any other the tree works through
+the registered torch op and says so once.
 """
 from __future__ import annotations
 

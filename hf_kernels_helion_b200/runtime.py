@@ -51,15 +51,21 @@ def status_word(device: torch.device) -> torch.Tensor:
     return w
 
 
-# csrc/torch_call.cpp, bound to the loaded library on the first call with a CUDA tensor
+# csrc/torch_call.cpp, bound to the loaded library on the first call with a CUDA tensor; None also where there is none
+# that this process can use
 native = None
+_native_missing = False
 
 
 def native_for(t):
-    """The native call module, or None for what is not a CUDA tensor (the Python path reports that)."""
-    global native
-    if native is None and isinstance(t, torch.Tensor) and t.is_cuda:
+    """The native call module; None where it cannot be used, and for what is not a CUDA tensor (the Python path reports
+    that)."""
+    global native, _native_missing
+    if native is None and not _native_missing and isinstance(t, torch.Tensor) and t.is_cuda:
         mod = _lib.load_native()
+        if mod is None:
+            _native_missing = True
+            return None
         for idx, w in list(_status_words.items()):
             mod.set_status(idx, w.data_ptr())
         native = mod

@@ -104,3 +104,35 @@ def test_shard_bounds():
     Bs = torch.arange(4 * 1).reshape(4, 1)
     b, bs = tp.shard_weight(B, Bs, 2, 1)
     assert torch.equal(b, B[256:]) and torch.equal(bs, Bs[2:])
+
+
+def test_native_module_is_optional(lib, monkeypatch):
+    """Without a native call module that this torch and this Python can use, the calls keep the way through the registered ops;
+    one that was built for others is never called."""
+    import sys
+    import types
+
+    from hf_kernels_helion_b200 import _lib
+
+    name = "hf_kernels_helion_b200._torch_call"
+    monkeypatch.delattr(pkg, "_torch_call", raising=False)
+    monkeypatch.setitem(sys.modules, name, None)                     # no file, or one that does not load
+    with pytest.warns(RuntimeWarning, match="does not load"):
+        assert _lib.load_native() is None
+
+    def never(*args):
+        raise AssertionError("called")
+
+    for other in (types.SimpleNamespace(bind=never, built_for="torch 1.0, Python 2.7"), types.SimpleNamespace(bind=never)):
+        monkeypatch.setitem(sys.modules, name, other)
+        monkeypatch.setattr(pkg, "_torch_call", other, raising=False)
+        with pytest.warns(RuntimeWarning, match="was built for"):
+            assert _lib.load_native() is None
+
+
+def test_native_module_is_rebuilt_for_another_torch(lib, monkeypatch):
+    from hf_kernels_helion_b200 import _lib, build
+
+    assert not build.is_stale()
+    monkeypatch.setattr(_lib, "native_tag", lambda: "torch 1.0, Python 2.7")
+    assert build.is_stale()

@@ -181,3 +181,22 @@ def test_other_threads_run_while_a_call_is_in_the_library(device, operands, tmp_
         _lib.load_native()      # binds the library again
     assert results == [True] * len(calls)
     assert torch.equal(_native(*operands), runtime.gemm(A, B, As, Bs, 128, 128, torch.float32))
+
+
+def test_calls_work_without_the_module(device, operands, monkeypatch):
+    """No module that fits (warned about once): the registered ops, the same bits."""
+    from hf_kernels_helion_b200 import _lib
+
+    A, B, As, Bs = operands
+    want = _native(*operands)
+    x = torch.randn(48, 512, device=device).to(torch.bfloat16)
+    q, s = runtime.native.act_quant(x, 128)
+    tried = []
+    monkeypatch.setattr(runtime, "native", None)
+    monkeypatch.setattr(runtime, "_native_missing", False)
+    monkeypatch.setattr(_lib, "load_native", lambda: tried.append(1))
+    for _ in range(2):
+        assert torch.equal(pkg.w8a8_block_fp8_matmul(A, B, As, Bs, [128, 128]), want)
+        rq, rs = pkg.fp8_act_quant(x)
+        assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(s, rs)
+    assert tried == [1] and runtime.native is None

@@ -65,3 +65,17 @@ print('ok')
 """
     res = _run(root, code)
     assert res.returncode == 0 and "ok" in res.stdout, res.stdout + res.stderr
+
+
+def test_tree_carries_the_native_call_module_and_works_without_it(tmp_path):
+    """The module serves the torch and the Python it was built for; without it the tree imports and says what it uses instead."""
+    root = _make(tmp_path)
+    assert (root / "_torch_call.so").exists()
+    code = ("import warnings; warnings.simplefilter('error')\n"
+            "import finegrained_fp8_helion as k\n"
+            "lib = __import__('sys').modules[k.w8a8_block_fp8_matmul.__module__].runtime._lib\n")
+    res = _run(root, code + "assert lib.load_native().built_for == lib.native_tag()\nprint('ok')")
+    assert res.returncode == 0 and "ok" in res.stdout, res.stderr
+    (root / "_torch_call.so").unlink()
+    res = _run(root, code + "warnings.simplefilter('ignore')\nassert lib.load_native() is None\nprint('ok')")
+    assert res.returncode == 0 and "ok" in res.stdout, res.stderr
