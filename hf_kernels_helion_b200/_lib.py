@@ -61,11 +61,15 @@ SIGNATURES = {
 _lib = None
 
 
+def is_built() -> bool:
+    return _lib is not None or LIB_PATH.exists()
+
+
 def load():
     """Load the library once; raise if it has not been built."""
     global _lib
     if _lib is None:
-        if not LIB_PATH.exists():
+        if not is_built():
             raise RuntimeError(
                 f"{LIB_PATH} is missing: build it with `python -m hf_kernels_helion_b200.build` "
                 "(there is no non-CUDA fallback)")

@@ -58,10 +58,11 @@ _native_missing = False
 
 
 def native_for(t):
-    """The native call module; None where it cannot be used, and for what is not a CUDA tensor (the Python path reports
-    that)."""
+    """The native call module; None where it cannot be used, for what is not a plain CUDA tensor (the Python path
+    handles or reports that), and while there is no library: what needs it says so, and tracing does not."""
     global native, _native_missing
-    if native is None and not _native_missing and isinstance(t, torch.Tensor) and t.is_cuda:
+    if (native is None and not _native_missing and type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda
+            and _lib.is_built()):
         mod = _lib.load_native()
         if mod is None:
             _native_missing = True

@@ -136,3 +136,24 @@ def test_native_module_is_rebuilt_for_another_torch(lib, monkeypatch):
     assert not build.is_stale()
     monkeypatch.setattr(_lib, "native_tag", lambda: "torch 1.0, Python 2.7")
     assert build.is_stale()
+
+
+def test_fake_cuda_tensors_need_no_library(monkeypatch, tmp_path):
+    """Tracing with fake CUDA tensors gives shapes and types where the library has not been built."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from hf_kernels_helion_b200 import _lib, deep_gemm
+
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "libb200fp8.so")
+    monkeypatch.setattr(runtime, "native", None)
+    monkeypatch.setattr(runtime, "_native_missing", False)
+    with FakeTensorMode():
+        A, B, As, Bs = [t.to("cuda") for t in _args(5, 256, 384)]
+        out = pkg.w8a8_block_fp8_matmul(A, B, As, Bs, [128, 128], torch.bfloat16)
+        assert out.shape == (5, 256) and out.dtype == torch.bfloat16 and out.is_cuda
+        q, s = pkg.fp8_act_quant(torch.empty(5, 384, dtype=torch.bfloat16, device="cuda"))
+        assert q.shape == (5, 384) and q.dtype == FP8 and s.shape == (5, 3)
+        out = deep_gemm.gemm_fp8_fp8_bf16_nt(A, B, As, Bs.repeat_interleave(128, 0))
+        assert out.shape == (5, 256) and out.dtype == torch.bfloat16
+    assert runtime.native is None and not runtime._native_missing
