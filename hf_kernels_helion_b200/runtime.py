@@ -44,8 +44,8 @@ def status_word(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     w = _status_words.get(idx)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
+        # (of two threads' words one stays, and both of them and the native module use that one)
+        w = _status_words.setdefault(idx, torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx)))
         if native is not None:
             native.set_status(idx, w.data_ptr())
     return w
@@ -67,9 +67,9 @@ def native_for(t):
         if mod is None:
             _native_missing = True
             return None
+        native = mod   # first, so that a word made from here on is told by the thread that makes it
         for idx, w in list(_status_words.items()):
             mod.set_status(idx, w.data_ptr())
-        native = mod
     return native
 
 

@@ -157,3 +157,46 @@ def test_fake_cuda_tensors_need_no_library(monkeypatch, tmp_path):
         out = deep_gemm.gemm_fp8_fp8_bf16_nt(A, B, As, Bs.repeat_interleave(128, 0))
         assert out.shape == (5, 256) and out.dtype == torch.bfloat16
     assert runtime.native is None and not runtime._native_missing
+
+
+def test_two_first_calls_agree_on_the_status_word(monkeypatch):
+    """Two threads' first calls on a device: one word for both and for the native call module. A word that only one of them
+    knew would be freed while the module still pointed kernels at it."""
+    import types
+
+    told, words, theirs = {}, {}, torch.zeros(1, dtype=torch.int32)
+
+    def zeros(*args, **kwargs):      # the other thread is done first while this one allocates
+        words[5] = theirs
+        return torch.ones(1, dtype=torch.int32)
+
+    monkeypatch.setattr(runtime, "_status_words", words)
+    monkeypatch.setattr(runtime, "native", types.SimpleNamespace(set_status=told.__setitem__))
+    monkeypatch.setattr(runtime, "torch", types.SimpleNamespace(zeros=zeros, int32=torch.int32, device=torch.device))
+    assert runtime.status_word(torch.device("cuda", 5)) is theirs and words == {5: theirs}
+    assert told == {5: theirs.data_ptr()}
+
+
+def test_native_module_learns_of_every_status_word(monkeypatch):
+    """A word that another thread makes while the module is being set up."""
+    import types
+
+    told, theirs = {}, torch.zeros(1, dtype=torch.int32)
+
+    class Words(dict):
+        def items(self):             # the other thread makes its word once these have been listed
+            listed = list(super().items())
+            self[7] = theirs
+            if runtime.native is not None:
+                runtime.native.set_status(7, theirs.data_ptr())
+            return listed
+
+    module = types.SimpleNamespace(set_status=told.__setitem__)
+    monkeypatch.setattr(runtime, "_status_words", Words())
+    monkeypatch.setattr(runtime, "native", None)
+    monkeypatch.setattr(runtime, "_native_missing", False)
+    monkeypatch.setattr(runtime._lib, "load_native", lambda: module)
+    monkeypatch.setattr(runtime._lib, "is_built", lambda: True)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
+    assert runtime.native_for(torch.zeros(1)) is module
+    assert told == {7: theirs.data_ptr()}
