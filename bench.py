@@ -17,6 +17,7 @@ Prints ONE JSON line on rank 0.  For N > 1 launch with torchrun, one rank per GP
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import statistics
@@ -612,13 +613,19 @@ def main_ours(args):
         fp8_peak = 2.0 * peaks["bf16_tflops"]
         gemm_flops = 2.0 * M * n_local * K
         achieved = gemm_flops / (gemm_ms * 1e-3) / 1e12
-        variant = _lib.load().b200fp8_gemm_pick_variant(M, n_local, K)
+        call = _lib.CALL_ONE if world == 1 or args.exchange == "nccl" else \
+            _lib.CALL_MULTICAST if args.exchange == "multimem" else _lib.CALL_SEVERAL
+        shared = ctypes.c_int(1)
+        variant = _lib.load().b200fp8_gemm_auto_form(M, n_local, K, call, ctypes.byref(shared))
         # (the 256-wide forms stage their output and store it by TMA: the *_multi_kernel instantiations, one destination at N = 1)
-        kernel = {1: "gemm_tile_kernel<128>", 2: "gemm_tile_multi_kernel<256>", 3: "gemm_streamk_kernel",
-                  4: "gemm_tile_kernel<256> with tail split-K", 5: "gemm_pair_multi_kernel<false>",
+        kernel = {1: "gemm_tile_kernel<128>", 2: "gemm_tile_multi_kernel<256>", 4: "gemm_tile_kernel<256> with tail split-K",
                   6: "gemm_pair_multi_kernel<true>", 7: "gemm_pair_multi_sk_kernel"}[variant]
-        if world > 1 and args.exchange == "fused" and variant == 2 and M > 128:
-            kernel = "gemm_pair_multi_kernel<true>"   # several destinations: AUTO takes the pair form whenever M > 128
+        if shared.value > 1:
+            kernel = f"gemm_cluster_kernel, {shared.value} CTAs a tile"
+        elif call == _lib.CALL_MULTICAST:
+            kernel = f"gemm_tile_mc_kernel<{128 * variant}>"
+        elif call == _lib.CALL_SEVERAL and variant == 1:
+            kernel = "gemm_tile_multi_kernel<128>"
         # DRAM bytes of one GEMM launch at 1 GPU, from one profiler capture of this kernel on this shape
         # (dram__bytes_read.sum / dram__bytes_write.sum); at N > 1 scaled by the share of the weight and of
         # the output a rank touches (A is read whole by every rank). Not re-measured by this run.
@@ -663,7 +670,7 @@ def main_ours(args):
             # pass where AUTO takes such a form; + the barrier kernel of the fused exchange (NCCL's all-gather and the
             # slot -> [M,N] copy are not counted: not ours)
             "gpu_launches": steps * (2 + (1 if world > 1 and args.exchange != "nccl" else 0)
-                                     + (1 if variant in (4, 7) and (world == 1 or args.exchange == "nccl") else 0)
+                                     + (1 if variant in (4, 7) else 0)
                                      + (1 if world > 1 and args.exchange == "fused" else 0)),
             "roofline": {"bound": "tensor", "kernel": kernel, "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp8_peak, "traffic": traffic,

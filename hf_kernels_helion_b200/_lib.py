@@ -19,6 +19,7 @@ VARIANT_AUTO, VARIANT_TILE128, VARIANT_TILE256, VARIANT_STREAMK, VARIANT_TILE256
 VARIANT_PAIR256, VARIANT_PAIR256_SPLIT = 5, 6
 VARIANT_NAMES = {"auto": 0, "tile128": 1, "tile256": 2, "streamk": 3, "tile256_sk": 4, "pair256": 5, "pair256_split": 6,
                  "pair256_split_sk": 7}
+CALL_ONE, CALL_ROWSCALE, CALL_SEVERAL, CALL_MULTICAST = 0, 1, 2, 3
 
 # name -> (restype, argtypes); mirrors include/b200fp8.h one to one
 SIGNATURES = {
@@ -49,6 +50,7 @@ SIGNATURES = {
     "b200fp8_ipc_open": (c_int, [c_void_p, c_void_p]),
     "b200fp8_ipc_close": (c_int, [c_void_p]),
     "b200fp8_gemm_workspace_bytes": (c_int64, [c_int64, c_int64, c_int64, c_int]),
+    "b200fp8_gemm_auto_form": (c_int, [c_int64, c_int64, c_int64, c_int, c_void_p]),
     "b200fp8_gemm_pick_variant": (c_int, [c_int64, c_int64, c_int64]),
     "b200fp8_gemm_pair_clusters": (c_int, []),
     "b200fp8_gemm_decode_static": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64,

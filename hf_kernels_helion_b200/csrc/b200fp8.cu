@@ -20,12 +20,16 @@ using namespace b200fp8;
 
 constexpr int kMaxDevices = 64;
 
-struct DeviceInfo {
-  std::atomic<int> ready{0};
-  int cc_major = 0;
+// What the choice of a form depends on besides the shape.
+struct Limits {
   int sm_count = 0;
   int pair_clusters = 0;   // CTA pairs of the pair kernels that can be resident at once
   int clusters[kClusterMax + 1] = {};   // clusters of c CTAs of gemm_cluster_kernel that can be resident at once
+};
+
+struct DeviceInfo : Limits {
+  std::atomic<int> ready{0};
+  int cc_major = 0;
 };
 DeviceInfo g_dev[kMaxDevices];
 std::mutex g_mutex;
@@ -166,12 +170,19 @@ int device_info(const DeviceInfo** out) {
   return B200FP8_OK;
 }
 
-int sm_count_or_default() {
+// For the queries: the current device's limits; without a device those of a B200, 148 SMs and as many clusters as they
+// hold, but no CTA pairs.
+Limits limits_or_default() {
   const DeviceInfo* d = nullptr;
-  if (device_info(&d) == B200FP8_OK) return d->sm_count;
+  if (device_info(&d) == B200FP8_OK) return *d;
   cudaGetLastError();
-  return 148;  // B200
+  Limits l;
+  l.sm_count = 148;
+  for (int c = 2; c <= kClusterMax; ++c) l.clusters[c] = l.sm_count / c;
+  return l;
 }
+
+int sm_count_or_default() { return limits_or_default().sm_count; }
 
 EncodeTiledFn encode_fn() {
   EncodeTiledFn fn = g_encode.load(std::memory_order_acquire);
@@ -438,10 +449,6 @@ Pick pick_form(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   return best;
 }
 
-int pick_variant(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
-  return pick_form(M, N, K, sm_count, pairs).variant;
-}
-
 // CTAs per tile (2..8) for products whose 128 x 128 tiles leave SMs idle: the K blocks of a tile are cut over a cluster
 // (gemm_cluster_kernel), as far as all clusters are resident at once. 1: another form is estimated to be faster.
 // Cutting costs 1-2 us (two cluster barriers and the addition through distributed shared memory), so that products of
@@ -485,6 +492,50 @@ Pick pick_rowb(int64_t M, int64_t N, int64_t K, int sm_count, int pairs) {
   if (t128 <= t_pair && t128 <= t_sk) return {B200FP8_VARIANT_TILE128, 8.0 + t128};
   if (t_sk < t_pair) return {B200FP8_VARIANT_PAIR256_SPLIT_SK, 8.0 + t_sk};
   return {B200FP8_VARIANT_PAIR256_SPLIT, 8.0 + t_pair};
+}
+
+int64_t partial_bytes(int variant, int64_t M, int64_t N, int64_t K, const Limits& lim) {
+  if (variant == B200FP8_VARIANT_TILE256_SK) return tile_sk_plan(M, N, K, lim.sm_count).partial_bytes;
+  if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK) return pair_sk_plan(M, N, K, lim.pair_clusters).partial_bytes;
+  return 0;
+}
+
+int without_split_tail(int variant) {
+  if (variant == B200FP8_VARIANT_TILE256_SK) return B200FP8_VARIANT_TILE256;
+  if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK) return B200FP8_VARIANT_PAIR256_SPLIT;
+  return variant;
+}
+
+// The form AUTO runs, decided here for the launches and for every query: a variant, and with
+// B200FP8_VARIANT_TILE128 the CTAs that share a tile. call: B200FP8_CALL_*; staged: the rows of every destination are
+// multiples of 16 bytes (only then do the pair forms pay, which stage their output).
+struct Form {
+  int variant;
+  int cluster;
+};
+
+Form auto_form(int64_t M, int64_t N, int64_t K, int call, bool staged, const Limits& lim) {
+  if (call == B200FP8_CALL_SEVERAL || call == B200FP8_CALL_MULTICAST) {
+    const int pairs = call == B200FP8_CALL_SEVERAL ? lim.pair_clusters : 0;
+    const int variant = without_split_tail(pick_form(M, N, K, lim.sm_count, pairs).variant);
+    // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room for a second set of
+    // output staging buffers, which keeps NVLink busy through the next tile's K loop
+    // (2 GPUs, 8192 x 18432 x 7168: 0.596 vs 0.608 ms for the unsplit form)
+    if (M > 128 && pairs > 0 && variant == B200FP8_VARIANT_TILE256) return {B200FP8_VARIANT_PAIR256_SPLIT, 1};
+    return {variant, 1};
+  }
+  const bool rowb = call == B200FP8_CALL_ROWSCALE;
+  const int pairs = staged ? lim.pair_clusters : 0;
+  const Pick p = rowb ? pick_rowb(M, N, K, lim.sm_count, pairs) : pick_form(M, N, K, lim.sm_count, pairs);
+  const int cluster = cluster_split(M, N, K, lim.clusters, p.us, rowb);
+  return {cluster > 1 ? B200FP8_VARIANT_TILE128 : p.variant, cluster};
+}
+
+// The partial tiles of whatever AUTO may run for this shape, with a destination that can be staged and with one that can't.
+int64_t auto_partial_bytes(int64_t M, int64_t N, int64_t K, int call, const Limits& lim) {
+  const int64_t a = partial_bytes(auto_form(M, N, K, call, true, lim).variant, M, N, K, lim);
+  const int64_t b = partial_bytes(auto_form(M, N, K, call, false, lim).variant, M, N, K, lim);
+  return a > b ? a : b;
 }
 
 // Whether the GEMM kernel reads the token scales (and, with up to 16 rows, A) where they are instead of copies that a
@@ -759,36 +810,26 @@ int64_t b200fp8_streamk_grid(int64_t M, int64_t N, int64_t K) {
   return streamk_plan(M, N, K, sm_count_or_default()).grid;
 }
 
-int b200fp8_gemm_pair_clusters(void) {
-  const DeviceInfo* d = nullptr;
-  if (device_info(&d) != B200FP8_OK) {
-    cudaGetLastError();
-    return 0;
-  }
-  return d->pair_clusters;
+int b200fp8_gemm_pair_clusters(void) { return limits_or_default().pair_clusters; }
+
+int b200fp8_gemm_auto_form(int64_t M, int64_t N, int64_t K, int call, int* ctas_per_tile) {
+  if (M < 1 || N < 1 || K < 1) return -B200FP8_ERR_SHAPE;
+  if (call < B200FP8_CALL_ONE || call > B200FP8_CALL_MULTICAST) return -B200FP8_ERR_VARIANT;
+  const Form f = auto_form(M, N, K, call, true, limits_or_default());
+  if (ctas_per_tile != nullptr) *ctas_per_tile = f.cluster;
+  return f.variant;
 }
 
 int b200fp8_gemm_pick_variant(int64_t M, int64_t N, int64_t K) {
-  return pick_variant(M, N, K, sm_count_or_default(), b200fp8_gemm_pair_clusters());
+  return auto_form(M, N, K, B200FP8_CALL_ONE, true, limits_or_default()).variant;
 }
 
 int64_t b200fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int variant) {
   if (M < 0 || N < 0 || K < 0) return -static_cast<int64_t>(B200FP8_ERR_SHAPE);
   const int sms = sm_count_or_default();
   if (M == 0 || N == 0 || K == 0) return (variant >= B200FP8_VARIANT_AUTO && variant <= B200FP8_VARIANT_PAIR256_SPLIT_SK) ? 0 : -static_cast<int64_t>(B200FP8_ERR_VARIANT);
-  if (variant == B200FP8_VARIANT_AUTO) {
-    // whatever AUTO may resolve to for this shape, with or without CTA pairs (a destination that cannot
-    // take 16-byte rows falls back to the single-CTA choice)
-    int64_t need = tile_workspace_bytes(M, K);
-    const int v1 = pick_variant(M, N, K, sms, 0);
-    if (v1 == B200FP8_VARIANT_TILE256_SK) need = tile_workspace_bytes(M, K) + tile_sk_plan(M, N, K, sms).partial_bytes;
-    const int pairs = b200fp8_gemm_pair_clusters();
-    if (pairs > 0 && pick_variant(M, N, K, sms, pairs) == B200FP8_VARIANT_PAIR256_SPLIT_SK) {
-      const int64_t np = tile_workspace_bytes(M, K) + pair_sk_plan(M, N, K, pairs).partial_bytes;
-      need = np > need ? np : need;
-    }
-    return need;
-  }
+  if (variant == B200FP8_VARIANT_AUTO)
+    return tile_workspace_bytes(M, K) + auto_partial_bytes(M, N, K, B200FP8_CALL_ONE, limits_or_default());
   if (variant == B200FP8_VARIANT_TILE128 || variant == B200FP8_VARIANT_TILE256 ||
       variant == B200FP8_VARIANT_PAIR256 || variant == B200FP8_VARIANT_PAIR256_SPLIT)
     return tile_workspace_bytes(M, K);
@@ -878,38 +919,26 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
   }
   if (M > 0x7FFFFF00 || N > 0x7FFFFF00 || K > 0x7FFFFF00) return B200FP8_ERR_TOO_LARGE;
 
-  const bool auto_variant = variant == B200FP8_VARIANT_AUTO;
-  // (the pair form only pays with the staged output: a destination that cannot take 16-byte rows gets the single-CTA choice)
-  double auto_us = 0.0;
-  if (auto_variant) {
-    const Pick p = pick_form(M, N, K, dev->sm_count, (staged && !mc && !fq.rowb) ? dev->pair_clusters : 0);
-    variant = p.variant;
-    auto_us = p.us;
-  }
-  if (fq.rowb) {
-    const Pick p = pick_rowb(M, N, K, dev->sm_count, staged ? dev->pair_clusters : 0);
-    variant = p.variant;
-    auto_us = p.us;
-    // (a workspace without room for the partial tiles: the same tiles without the split tail)
-    if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK &&
-        static_cast<int64_t>(workspace_bytes) < tile_workspace_bytes(M, K) + bst_bytes(N, K) +
-                                                    pair_sk_plan(M, N, K, dev->pair_clusters).partial_bytes)
-      variant = B200FP8_VARIANT_PAIR256_SPLIT;
-  }
   const bool multi = n_dst > 1 || mc;
-  const int cluster =
-      (auto_variant || fq.rowb) && !multi ? cluster_split(M, N, K, dev->clusters, auto_us, fq.rowb) : 1;
-  if (cluster > 1) variant = B200FP8_VARIANT_TILE128;
   if (fq.rowb && (multi || fused_q)) return B200FP8_ERR_VARIANT;
-  // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room
-  // for a second set of output staging buffers, which keeps NVLink busy through the next tile's K loop
+  int cluster = 1;
+  if (variant == B200FP8_VARIANT_AUTO || fq.rowb) {
+    const int call = fq.rowb ? B200FP8_CALL_ROWSCALE
+                     : mc    ? B200FP8_CALL_MULTICAST
+                             : n_dst > 1 ? B200FP8_CALL_SEVERAL : B200FP8_CALL_ONE;
+    const Form f = auto_form(M, N, K, call, staged, *dev);
+    variant = f.variant;
+    cluster = f.cluster;
+    // (a workspace without room for the partial tiles: the same tiles without the split tail)
+    if (fq.rowb && static_cast<int64_t>(workspace_bytes) <
+                       tile_workspace_bytes(M, K) + bst_bytes(N, K) + partial_bytes(variant, M, N, K, *dev))
+      variant = without_split_tail(variant);
+  }
   if (multi && variant == B200FP8_VARIANT_TILE256_SK) variant = B200FP8_VARIANT_TILE256;
   // the K ranges of the pair split-K form leave through the fix-up pass, which writes one destination,
   // and its whole tiles through the staging area
   if (variant == B200FP8_VARIANT_PAIR256_SPLIT_SK && (multi || !staged || dev->pair_clusters < 1))
     variant = B200FP8_VARIANT_PAIR256_SPLIT;
-  if (auto_variant && n_dst > 1 && !mc && M > 128 && dev->pair_clusters > 0 && variant == B200FP8_VARIANT_TILE256)
-    variant = B200FP8_VARIANT_PAIR256_SPLIT;   // (2 GPUs, 8192 x 18432 x 7168: 0.596 vs 0.608 ms for the unsplit form)
   const bool pair = variant == B200FP8_VARIANT_PAIR256 || variant == B200FP8_VARIANT_PAIR256_SPLIT ||
                     variant == B200FP8_VARIANT_PAIR256_SPLIT_SK;
   if (pair && mc) return B200FP8_ERR_VARIANT;
@@ -1087,9 +1116,8 @@ int b200fp8_gemm_rowscale(const void* A, const void* B, const float* As, const f
 int64_t b200fp8_gemm_rowscale_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M < 0 || N < 0 || K < 0) return -static_cast<int64_t>(B200FP8_ERR_SHAPE);
   if (M == 0 || N == 0 || K == 0) return 0;
-  const int pairs = b200fp8_gemm_pair_clusters();
-  const bool sk = pick_rowb(M, N, K, sm_count_or_default(), pairs).variant == B200FP8_VARIANT_PAIR256_SPLIT_SK;
-  return tile_workspace_bytes(M, K) + bst_bytes(N, K) + (sk ? pair_sk_plan(M, N, K, pairs).partial_bytes : 0);
+  return tile_workspace_bytes(M, K) + bst_bytes(N, K) +
+         auto_partial_bytes(M, N, K, B200FP8_CALL_ROWSCALE, limits_or_default());
 }
 
 int b200fp8_linear(const void* x_bf16, const void* B, const float* Bs, void* C, int64_t M, int64_t N, int64_t K,
@@ -1109,16 +1137,8 @@ int64_t b200fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K, int vari
   if (M < 0 || N < 0 || K < 0) return -static_cast<int64_t>(B200FP8_ERR_SHAPE);
   if (M == 0 || N == 0 || K == 0) return 0;
   const int sms = sm_count_or_default();
-  if (variant == B200FP8_VARIANT_AUTO) {
-    int64_t extra = 0;
-    if (pick_variant(M, N, K, sms, 0) == B200FP8_VARIANT_TILE256_SK) extra = tile_sk_plan(M, N, K, sms).partial_bytes;
-    const int pairs = b200fp8_gemm_pair_clusters();
-    if (pairs > 0 && pick_variant(M, N, K, sms, pairs) == B200FP8_VARIANT_PAIR256_SPLIT_SK) {
-      const int64_t ep = pair_sk_plan(M, N, K, pairs).partial_bytes;
-      extra = ep > extra ? ep : extra;
-    }
-    return linear_prefix_bytes(M, K) + extra;
-  }
+  if (variant == B200FP8_VARIANT_AUTO)
+    return linear_prefix_bytes(M, K) + auto_partial_bytes(M, N, K, B200FP8_CALL_ONE, limits_or_default());
   if (variant == B200FP8_VARIANT_TILE128 || variant == B200FP8_VARIANT_TILE256 ||
       variant == B200FP8_VARIANT_PAIR256 || variant == B200FP8_VARIANT_PAIR256_SPLIT)
     return linear_prefix_bytes(M, K);

@@ -251,7 +251,19 @@ int b200fp8_ipc_close(void* base);
 /* Bytes of workspace b200fp8_gemm needs for this call (0 when none). Negative = error status, negated. */
 int64_t b200fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int variant);
 
-/* The variant B200FP8_VARIANT_AUTO resolves to for this shape on the current device. */
+/*
+ * The variant B200FP8_VARIANT_AUTO resolves to for this shape on the current device, for a destination whose rows are
+ * multiples of 16 bytes; and how many CTAs (a cluster of 2..8) share each tile along K, which only
+ * B200FP8_VARIANT_TILE128 has, otherwise 1. `call` says whose AUTO: b200fp8_gemm and b200fp8_linear (ONE),
+ * b200fp8_gemm_rowscale, b200fp8_gemm_scatter with several destinations, b200fp8_gemm_multicast. Negative = error
+ * status, negated. Without a device: a B200 that runs no CTA pairs. pick_variant is the variant of ONE. (The reference's
+ * counterpart is the choice among its tuned configs, torch-ext/finegrained_fp8_helion/_helion_aot_fp8_cuda_sm100.py:13-28.)
+ */
+#define B200FP8_CALL_ONE 0
+#define B200FP8_CALL_ROWSCALE 1
+#define B200FP8_CALL_SEVERAL 2
+#define B200FP8_CALL_MULTICAST 3
+int b200fp8_gemm_auto_form(int64_t M, int64_t N, int64_t K, int call, int* ctas_per_tile);
 int b200fp8_gemm_pick_variant(int64_t M, int64_t N, int64_t K);
 
 /*

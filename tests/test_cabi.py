@@ -209,3 +209,34 @@ def test_peer_barrier_wait_runs_out_cleanly(lib, device):
     out = runtime.gemm(A.to(device), B.to(device), As.to(device), Bs.to(device), 128, 128, torch.float32)
     runtime.check_device_status(device)
     assert oracle.max_err_over_rms(out.cpu(), oracle.gemm_dequant(A, B, As, Bs)) <= 1e-4
+
+
+def test_queries_name_the_form_that_runs(lib):
+    """One decision for the launches and the queries: a product whose tiles are shared by clusters is one of 128 x 128 tiles, and
+    its workspace has no partial tiles in it."""
+    ONE, ROWSCALE, SEVERAL, MULTICAST = 0, 1, 2, 3
+    shared = ctypes.c_int(0)
+
+    def form(M, N, K, call):
+        return lib.b200fp8_gemm_auto_form(M, N, K, call, ctypes.byref(shared)), shared.value
+
+    for M, N, K in [(512, 512, 8192), (4, 2560, 2048), (130, 384, 2048)]:
+        variant, ctas = form(M, N, K, ONE)
+        assert variant == 1 and 2 <= ctas <= 8
+        assert lib.b200fp8_gemm_pick_variant(M, N, K) == 1
+        kb, m_pad = -(-K // 128), -(-M // 128) * 128
+        scales = kb * m_pad * 4
+        assert lib.b200fp8_gemm_workspace_bytes(M, N, K, 0) == scales + (16 * K if M <= 16 else 0)
+        assert lib.b200fp8_linear_workspace_bytes(M, N, K, 0) == scales + max(M, 16) * K
+    variant, ctas = form(300, 264, 16400, ROWSCALE)
+    assert variant == 1 and 2 <= ctas <= 8
+    assert lib.b200fp8_gemm_rowscale_workspace_bytes(300, 264, 16400) == 129 * 384 * 4 + 129 * 384 * 4
+    for M, N, K in [(8192, 18432, 7168), (16, 28672, 8192), (512, 512, 512)]:
+        for call in (ONE, ROWSCALE, SEVERAL, MULTICAST):
+            variant, ctas = form(M, N, K, call)
+            assert 1 <= variant <= 7 and ctas == 1
+            assert call == ONE or call == ROWSCALE or variant in (1, 2, 6)      # the fix-up pass writes one destination
+            assert call != ONE or variant == lib.b200fp8_gemm_pick_variant(M, N, K)
+    assert lib.b200fp8_gemm_auto_form(4, 2560, 2048, ONE, None) == 1
+    assert lib.b200fp8_gemm_auto_form(0, 2560, 2048, ONE, None) == -2
+    assert lib.b200fp8_gemm_auto_form(4, 2560, 2048, 4, None) == -5
