@@ -506,6 +506,26 @@ int without_split_tail(int variant) {
   return variant;
 }
 
+double wave_efficiency(int64_t tiles, int sms) {
+  return static_cast<double>(tiles) / static_cast<double>((tiles + sms - 1) / sms * sms);
+}
+
+// Several destinations (the N-sharded exchange), or one multicast address (no pairs). The estimates above are of single
+// destinations, whose last wave may be split and whose stores stay on the device: they do not say what an exchange takes,
+// which is bound by the links, so this rule is the one that exchanges over NVLink were measured with. 256-wide tiles move 25 %
+// fewer operand bytes per flop and are taken unless their last wave is much emptier, on CTA pairs beyond 128 rows: the
+// pair kernel's smaller pipeline stages leave room for a second set of output staging buffers, which keeps the links busy
+// through the next tile's K loop (2 GPUs, 8192 x 18432 x 7168: 0.596 ms, 0.608 for the pair form with whole K blocks; 4 GPUs
+// 0.538 against 0.540 for single CTAs).
+int pick_several(int64_t M, int64_t N, int sm_count, int pairs) {
+  if (M <= 128 || (M <= 256 && (N <= 128 || pairs < 1))) return N > 128 ? B200FP8_VARIANT_TILE256 : B200FP8_VARIANT_TILE128;
+  const int64_t num_m = (M + 127) / 128;
+  const double e128 = wave_efficiency(num_m * ((N + 127) / 128), sm_count);
+  const double e256 = wave_efficiency(num_m * ((N + 255) / 256), sm_count);
+  if (e256 * 1.15 < e128) return B200FP8_VARIANT_TILE128;
+  return pairs > 0 ? B200FP8_VARIANT_PAIR256_SPLIT : B200FP8_VARIANT_TILE256;
+}
+
 // The form AUTO runs, decided here for the launches and for every query: a variant, and with
 // B200FP8_VARIANT_TILE128 the CTAs that share a tile. call: B200FP8_CALL_*; staged: the rows of every destination are
 // multiples of 16 bytes (only then do the pair forms pay, which stage their output).
@@ -515,15 +535,8 @@ struct Form {
 };
 
 Form auto_form(int64_t M, int64_t N, int64_t K, int call, bool staged, const Limits& lim) {
-  if (call == B200FP8_CALL_SEVERAL || call == B200FP8_CALL_MULTICAST) {
-    const int pairs = call == B200FP8_CALL_SEVERAL ? lim.pair_clusters : 0;
-    const int variant = without_split_tail(pick_form(M, N, K, lim.sm_count, pairs).variant);
-    // Several destinations (the N-sharded exchange): the pair kernel's smaller pipeline stages leave room for a second set of
-    // output staging buffers, which keeps NVLink busy through the next tile's K loop
-    // (2 GPUs, 8192 x 18432 x 7168: 0.596 vs 0.608 ms for the unsplit form)
-    if (M > 128 && pairs > 0 && variant == B200FP8_VARIANT_TILE256) return {B200FP8_VARIANT_PAIR256_SPLIT, 1};
-    return {variant, 1};
-  }
+  if (call == B200FP8_CALL_SEVERAL || call == B200FP8_CALL_MULTICAST)
+    return {pick_several(M, N, lim.sm_count, call == B200FP8_CALL_SEVERAL ? lim.pair_clusters : 0), 1};
   const bool rowb = call == B200FP8_CALL_ROWSCALE;
   const int pairs = staged ? lim.pair_clusters : 0;
   const Pick p = rowb ? pick_rowb(M, N, K, lim.sm_count, pairs) : pick_form(M, N, K, lim.sm_count, pairs);

@@ -383,3 +383,50 @@ def test_auto_on_small_and_ragged_products(device, M, N, K):
     assert _rel(out16, A, B, As, Bs) <= 2.0 ** -8
     assert bool((half[:, 0] == 0).all()) and bool((half[:, N + 1:] == 0).all())
     runtime.check_device_status()
+
+
+def _several(M, N, sms, pairs):
+    """Which tiles an exchange runs on: as it was measured over NVLink, whatever single destinations take."""
+    def full(tiles):
+        return tiles / (-(-tiles // sms) * sms)
+
+    if M <= 128 or (M <= 256 and (N <= 128 or not pairs)):
+        return "tile256" if N > 128 else "tile128"
+    rows = -(-M // 128)
+    if full(rows * -(-N // 256)) * 1.15 < full(rows * -(-N // 128)):
+        return "tile128"
+    return "pair256_split" if pairs else "tile256"
+
+
+@pytest.mark.parametrize("M,N,K,n", [(1, 256, 512, 2), (64, 2560, 2048, 2), (128, 384, 1664, 3), (200, 128, 512, 2),
+                                     (200, 512, 640, 8), (512, 512, 2048, 2), (640, 4096, 1024, 2), (1000, 1288, 1168, 3),
+                                     (4096, 512, 256, 2)])
+def test_several_destinations(device, M, N, K, n):
+    """b200fp8_gemm_scatter into n local buffers, a column slice of each: every copy has the bits of the single-destination kernel
+    with those tiles, and nothing around the slices is touched."""
+    lib = _lib.load()
+    name = _several(M, N, torch.cuda.get_device_properties(device).multi_processor_count, lib.b200fp8_gemm_pair_clusters())
+    assert lib.b200fp8_gemm_auto_form(M, N, K, _lib.CALL_SEVERAL, None) == _lib.VARIANT_NAMES[name]
+    single = _several(M, N, torch.cuda.get_device_properties(device).multi_processor_count, 0)
+    assert lib.b200fp8_gemm_auto_form(M, N, K, _lib.CALL_MULTICAST, None) == _lib.VARIANT_NAMES[single]
+    A, B, As, Bs = _dev(oracle.make_quantised_inputs(M, N, K, M + N + K), device)
+    for dtype in (torch.bfloat16, torch.float32):
+        want = runtime.gemm(A, B, As, Bs, 128, 128, dtype, variant=name)
+        bufs = [torch.full((M + 2, N + 32 + 16 * d), 7.0, dtype=dtype, device=device) for d in range(n)]
+        slices = [b[1:M + 1, 16:16 + N] for b in bufs]
+        runtime.gemm_scatter(A, B, As, Bs, [s.data_ptr() for s in slices], [b.stride(0) for b in bufs], dtype)
+        runtime.check_device_status()
+        for b, s in zip(bufs, slices):
+            assert torch.equal(s, want)
+            s.fill_(7.0)
+            assert bool((b == 7.0).all())
+
+
+def test_several_destinations_rule_over_sizes(device):
+    """The same rule for every size, not only those that run here."""
+    lib = _lib.load()
+    sms, pairs = torch.cuda.get_device_properties(device).multi_processor_count, lib.b200fp8_gemm_pair_clusters()
+    for M in (1, 128, 129, 256, 257, 500, 640, 1611, 2545, 4096, 8192):
+        for N in (16, 128, 144, 512, 1920, 2304, 7000, 18432, 28672):
+            for call, p in ((_lib.CALL_SEVERAL, pairs), (_lib.CALL_MULTICAST, 0)):
+                assert lib.b200fp8_gemm_auto_form(M, N, 1024, call, None) == _lib.VARIANT_NAMES[_several(M, N, sms, p)], (M, N, call)
