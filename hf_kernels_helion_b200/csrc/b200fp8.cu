@@ -934,6 +934,9 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
 
   const bool multi = n_dst > 1 || mc;
   if (fq.rowb && (multi || fused_q)) return B200FP8_ERR_VARIANT;
+  // what every tile form needs of the workspace: the scale copy, the copy of A, and the copy of B's row scales
+  const int64_t prefix = fused_q ? linear_prefix_bytes(M, K) : tile_workspace_bytes(M, K);
+  const int64_t rowb_bytes = fq.rowb ? bst_bytes(N, K) : 0;
   int cluster = 1;
   if (variant == B200FP8_VARIANT_AUTO || fq.rowb) {
     const int call = fq.rowb ? B200FP8_CALL_ROWSCALE
@@ -943,8 +946,7 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
     variant = f.variant;
     cluster = f.cluster;
     // (a workspace without room for the partial tiles: the same tiles without the split tail)
-    if (fq.rowb && static_cast<int64_t>(workspace_bytes) <
-                       tile_workspace_bytes(M, K) + bst_bytes(N, K) + partial_bytes(variant, M, N, K, *dev))
+    if (static_cast<int64_t>(workspace_bytes) < prefix + rowb_bytes + partial_bytes(variant, M, N, K, *dev))
       variant = without_split_tail(variant);
   }
   if (multi && variant == B200FP8_VARIANT_TILE256_SK) variant = B200FP8_VARIANT_TILE256;
@@ -972,8 +974,7 @@ static int gemm_impl(bool mc, const void* A, const void* B, const float* As, con
       variant == B200FP8_VARIANT_TILE256_SK || pair) {
     const bool pair_sk = variant == B200FP8_VARIANT_PAIR256_SPLIT_SK;
     const bool sk = variant == B200FP8_VARIANT_TILE256_SK || pair_sk;
-    const int64_t prefix = fused_q ? linear_prefix_bytes(M, K) : tile_workspace_bytes(M, K);
-    const int64_t need = prefix + (sk ? skp.partial_bytes : 0) + (fq.rowb ? bst_bytes(N, K) : 0);
+    const int64_t need = prefix + (sk ? skp.partial_bytes : 0) + rowb_bytes;
     if (workspace == nullptr || static_cast<int64_t>(workspace_bytes) < need) return B200FP8_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return B200FP8_ERR_ALIGN;
     GemmArgs args;

@@ -121,9 +121,10 @@ int b200fp8_quant_weight(const void* w, void* q, float* s,
  * no-op; K == 0 writes zeros.
  *
  * `workspace` holds per-call scratch (room for a K-block-major copy of As for every variant, plus
- * the fp32 partial tiles of B200FP8_VARIANT_STREAMK); size it with
+ * the fp32 partial tiles of the forms that split K through memory); size it with
  * b200fp8_gemm_workspace_bytes for the same (M, N, K, variant), align it to 256 bytes. Its
- * contents need no initialisation.
+ * contents need no initialisation. (Where AUTO would split its last wave and the workspace holds
+ * only what B200FP8_VARIANT_TILE256 needs, the same tiles run without the split.)
  */
 int b200fp8_gemm(const void* A, const void* B, const float* As, const float* Bs, void* C,
                  int64_t M, int64_t N, int64_t K,

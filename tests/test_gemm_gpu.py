@@ -430,3 +430,44 @@ def test_several_destinations_rule_over_sizes(device):
         for N in (16, 128, 144, 512, 1920, 2304, 7000, 18432, 28672):
             for call, p in ((_lib.CALL_SEVERAL, pairs), (_lib.CALL_MULTICAST, 0)):
                 assert lib.b200fp8_gemm_auto_form(M, N, 1024, call, None) == _lib.VARIANT_NAMES[_several(M, N, sms, p)], (M, N, call)
+
+
+@pytest.mark.parametrize("M,N,K", [(131, 5248, 6400), (1000, 5120, 4096)])
+def test_auto_with_a_workspace_that_holds_no_partial_tiles(device, M, N, K):
+    """AUTO's choice of a split last wave asks for room for its partial tiles; a caller that has only what every tile form
+    needs gets the same tiles without the split, and only a smaller workspace is refused."""
+    lib = _lib.load()
+    A, B, As, Bs = _dev(oracle.make_quantised_inputs(M, N, K, M + N + K), device)
+    Bs_row = Bs.repeat_interleave(128, 0)[:N].contiguous()
+    x = torch.randn(M, K, device=device).to(torch.bfloat16)
+    kb = K // 128
+    out = torch.empty(M, N, device=device)
+    word, stream = runtime.status_word(device).data_ptr(), torch.cuda.current_stream(device).cuda_stream
+    plain = lib.b200fp8_gemm_workspace_bytes(M, N, K, _lib.VARIANT_TILE256)
+    assert lib.b200fp8_gemm_pick_variant(M, N, K) in (4, 7) and lib.b200fp8_gemm_workspace_bytes(M, N, K, 0) > plain
+    linear = lib.b200fp8_linear_workspace_bytes(M, N, K, _lib.VARIANT_TILE256)
+    rows = plain + kb * -(-N // 128) * 128 * 4
+    ws = torch.empty(max(linear, rows), dtype=torch.uint8, device=device)
+
+    def gemm(size):
+        return lib.b200fp8_gemm(A.data_ptr(), B.data_ptr(), As.data_ptr(), Bs.data_ptr(), out.data_ptr(), M, N, K, K, K, kb, kb,
+                                N, _lib.OUT_FP32, 0, ws.data_ptr(), size, word, stream)
+
+    def fused(size):
+        return lib.b200fp8_linear(x.data_ptr(), B.data_ptr(), Bs.data_ptr(), out.data_ptr(), M, N, K, K, K, kb, N,
+                                  _lib.OUT_FP32, 0, ws.data_ptr(), size, word, stream)
+
+    def rowscale(size):
+        return lib.b200fp8_gemm_rowscale(A.data_ptr(), B.data_ptr(), As.data_ptr(), Bs_row.data_ptr(), out.data_ptr(), M, N, K,
+                                         K, K, kb, kb, N, _lib.OUT_FP32, ws.data_ptr(), size, word, stream)
+
+    q, s = pkg.fp8_act_quant(x)
+    for call, size, want in ((gemm, plain, runtime.gemm(A, B, As, Bs, 128, 128, torch.float32, variant="tile256")),
+                             (fused, linear, runtime.gemm(q, B, s, Bs, 128, 128, torch.float32, variant="tile256")),
+                             (rowscale, rows, runtime.gemm_rowscale(A, B, As, Bs_row, 128, torch.float32))):
+        out.zero_()
+        assert call(size) == 0
+        runtime.check_device_status()
+        assert oracle.max_err_over_rms(out.cpu(), want.cpu()) <= 2e-6
+        assert call is rowscale or torch.equal(out, want)      # whole tiles add the K blocks in order, whichever form
+        assert call(size - 1) == 6                               # B200FP8_ERR_WORKSPACE
