@@ -738,7 +738,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
           for (int i = 0; i < 16; ++i) sv[i] = reinterpret_cast<const float4*>(sbt)[i];   // same address in all lanes: broadcast
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) sv[i] = __ldg(reinterpret_cast<const float4*>(sbt) + i);
+          for (int i = 0; i < 16; ++i) sv[i] = ld_global(reinterpret_cast<const float4*>(sbt) + i);
         }
         const uint32_t ts = it % TS;
         const uint32_t tph = (it / TS) & 1u;
@@ -865,26 +865,26 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
       auto load_as = [&](int kb, float (&sa)[PF]) {
         if (as_vec && kb + PF <= seg.kb_end) {
           if constexpr (PF == 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(as_col + kb));
+            const float4 v = ld_global(reinterpret_cast<const float4*>(as_col + kb));
             sa[0] = v.x;
             sa[1] = v.y;
             sa[PF - 2] = v.z;
             sa[PF - 1] = v.w;
           } else {
-            const float2 v = __ldg(reinterpret_cast<const float2*>(as_col + kb));
+            const float2 v = ld_global(reinterpret_cast<const float2*>(as_col + kb));
             sa[0] = v.x;
             sa[1] = v.y;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < PF; ++j) sa[j] = __ldg(as_col + (kb + j < seg.kb_end ? kb + j : kb_last) * as_step);
+          for (int j = 0; j < PF; ++j) sa[j] = ld_global(as_col + (kb + j < seg.kb_end ? kb + j : kb_last) * as_step);
         }
       };
       load_as(seg.kb_begin, sa_c);
 #pragma unroll
       for (int j = 0; j < PF; ++j) {
         const int k = seg.kb_begin + j < seg.kb_end ? seg.kb_begin + j : kb_last;
-        sb_c[j] = ROWB ? 1.f : __ldg(bs_row + k);
+        sb_c[j] = ROWB ? 1.f : ld_global(bs_row + k);
       }
       for (int kb0 = seg.kb_begin; ok && kb0 < seg.kb_end; kb0 += PF) {
         load_as(kb0 + PF, sa_n);
@@ -892,7 +892,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& tmap_a, const 
         for (int j = 0; j < PF; ++j) {
           int k = kb0 + PF + j;
           k = k < seg.kb_end ? k : kb_last;
-          sb_n[j] = ROWB ? 1.f : __ldg(bs_row + k);
+          sb_n[j] = ROWB ? 1.f : ld_global(bs_row + k);
         }
 #pragma unroll
         for (int j = 0; j < PF; ++j) {
@@ -1209,7 +1209,7 @@ gemm_tile_mc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // rows, rows >= M zero) and the scales K-block-major into AsT[kb][m_pad] (rows >= M zero).
 // K is a multiple of 128. Eight threads per 128-element group; groups = m_pad x K/128.
 __global__ void __launch_bounds__(256)
-tile_prep_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, uint8_t* __restrict__ Aq, int64_t ldq,
+tile_prep_quant_kernel(const __nv_bfloat16* x, int64_t ldx, uint8_t* __restrict__ Aq, int64_t ldq,
                        int64_t rows_q, float* __restrict__ AsT, int64_t M, int64_t m_pad, int num_kb) {
   // wait first, so that the GEMM kernel, which loads weights before it waits, starts after the kernel before this one
   pdl_wait();
@@ -1226,8 +1226,8 @@ tile_prep_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, uint8_t
   v[1] = make_uint4(0u, 0u, 0u, 0u);
   if (row < M) {
     const uint4* src = reinterpret_cast<const uint4*>(x + row * ldx + kg * 128 + sub * 16);
-    v[0] = __ldg(src);
-    v[1] = __ldg(src + 1);
+    v[0] = ld_global(src);
+    v[1] = ld_global(src + 1);
   }
   float amax = fmax_nan(amax8(v[0]), amax8(v[1]));
   amax = fmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
@@ -1251,7 +1251,7 @@ tile_prep_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, uint8_t
 // (fp32) row segments. Launched with programmatic stream serialisation: it may be scheduled
 // while the GEMM drains, and waits for it here before it reads.
 __global__ void __launch_bounds__(256)
-tile_sk_fixup_kernel(const float* __restrict__ partial, void* C, int64_t M, int64_t N, int num_kb, int64_t ldc,
+tile_sk_fixup_kernel(const float* partial, void* C, int64_t M, int64_t N, int num_kb, int64_t ldc,
                      int out_fp32, int num_m, int num_n, int sk_full, int sk_split, int sk_kb_per, int pair) {
   // pair != 0: the tiles are 256 rows tall and each K range was left by the two CTAs of a pair, rows
   // 0..127 in slot 2 u and rows 128..255 in slot 2 u + 1 of range u (grid.y = 8 instead of 4)
@@ -1277,7 +1277,7 @@ tile_sk_fixup_kernel(const float* __restrict__ partial, void* C, int64_t M, int6
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int c4 = cq * (QN / 4) + 2 * warp + i;
-        const float4 v = __ldg(reinterpret_cast<const float4*>(partial) + (static_cast<int64_t>(slot) * (BN / 4) + c4) * 128 + r0 + lane);
+        const float4 v = ld_global(reinterpret_cast<const float4*>(partial) + (static_cast<int64_t>(slot) * (BN / 4) + c4) * 128 + r0 + lane);
         sum[i].x += v.x;
         sum[i].y += v.y;
         sum[i].z += v.z;
@@ -1366,7 +1366,7 @@ struct ScaleCopy {
 //   A       (only when M <= 16) A_pad[16][lda_pad] = A with zero rows appended: TMA boxes over a
 //           tensor of fewer than 16 rows measured ~20 % slower on B200 than over 16 rows.
 __global__ void __launch_bounds__(256)
-tile_prep_kernel(const ScaleCopy first, const ScaleCopy second, int num_kb, const uint8_t* __restrict__ A,
+tile_prep_kernel(const ScaleCopy first, const ScaleCopy second, int num_kb, const uint8_t* A,
                  uint8_t* __restrict__ A_pad, int64_t M, int64_t K, int64_t lda, int64_t lda_pad) {
   // let the GEMM kernel that follows (launched with programmatic stream serialisation) start its prologue and its weight
   // loads once the kernel before this one is done; the warps that read what this grid writes wait for it
@@ -1383,7 +1383,7 @@ tile_prep_kernel(const ScaleCopy first, const ScaleCopy second, int num_kb, cons
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < M) {
         if (c + 16 <= K) {
-          v = __ldg(reinterpret_cast<const uint4*>(A + r * lda + c));
+          v = ld_global(reinterpret_cast<const uint4*>(A + r * lda + c));
         } else {
           uint8_t b[16];
 #pragma unroll
@@ -1405,7 +1405,7 @@ tile_prep_kernel(const ScaleCopy first, const ScaleCopy second, int num_kb, cons
   for (int i = 0; i < 32; i += 8) {
     const int64_t m = m0 + ty + i;
     const int kb = kb0 + tx;
-    t[ty + i][tx] = (m < s.rows && kb < num_kb) ? __ldg(s.src + m * s.ld + kb) : 0.f;
+    t[ty + i][tx] = (m < s.rows && kb < num_kb) ? ld_global(s.src + m * s.ld + kb) : 0.f;
   }
   __syncthreads();
 #pragma unroll

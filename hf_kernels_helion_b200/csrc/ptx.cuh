@@ -37,6 +37,33 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Loads for kernels that start before the kernel in front of them has ended: ordinary ones, in volatile asm, which the
+// compiler keeps below pdl_wait. __ldg and ld.global.nc are for data that nobody writes while the kernel runs, which the
+// operands of such a kernel are not, and the compiler may move them up past the wait.
+__device__ __forceinline__ float ld_global(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ float2 ld_global(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ float4 ld_global(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ uint4 ld_global(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // ----------------------------------------------------------------------------- CTA pairs (clusters of two)
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {

@@ -126,12 +126,12 @@ __device__ __forceinline__ void quant_vecs(const uint4 (&v)[NV], float scale, ui
 template <bool WIDE>
 __device__ __forceinline__ void load_32b(const void* p, uint4& lo, uint4& hi) {
   if constexpr (WIDE) {
-    asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
                  : "l"(p));
   } else {
-    lo = __ldg(static_cast<const uint4*>(p));
-    hi = __ldg(static_cast<const uint4*>(p) + 1);
+    lo = ld_global(static_cast<const uint4*>(p));
+    hi = ld_global(static_cast<const uint4*>(p) + 1);
   }
 }
 
@@ -144,7 +144,7 @@ __device__ __forceinline__ void load_32b(const void* p, uint4& lo, uint4& hi) {
 // 6.3 TB/s, the copy rate of the part).
 template <bool WIDE>
 __global__ void __launch_bounds__(256)
-quant_act_contig_kernel(const uint4* __restrict__ x, uint4* __restrict__ q, float* __restrict__ s,
+quant_act_contig_kernel(const uint4* x, uint4* __restrict__ q, float* __restrict__ s,
                         int64_t total_groups) {
   pdl_wait();
   pdl_trigger();
@@ -178,7 +178,7 @@ quant_act_contig_kernel(const uint4* __restrict__ x, uint4* __restrict__ q, floa
 // whenever the padded group count fits (its division is several times cheaper), 64 otherwise.
 template <typename Idx>
 __global__ void __launch_bounds__(256)
-quant_act_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ s, int64_t M,
+quant_act_kernel(const __nv_bfloat16* x, uint8_t* __restrict__ q, float* __restrict__ s, int64_t M,
                  int64_t K, int64_t ldx, int64_t ldq, int64_t lds) {
   pdl_wait();
   pdl_trigger();
@@ -199,8 +199,8 @@ quant_act_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, f
     v[0] = make_uint4(0u, 0u, 0u, 0u);
     v[1] = make_uint4(0u, 0u, 0u, 0u);
     const __nv_bfloat16* src = x + static_cast<int64_t>(row) * ldx + col;
-    if (has0) v[0] = __ldg(reinterpret_cast<const uint4*>(src));
-    if (has1) v[1] = __ldg(reinterpret_cast<const uint4*>(src + 8));
+    if (has0) v[0] = ld_global(reinterpret_cast<const uint4*>(src));
+    if (has1) v[1] = ld_global(reinterpret_cast<const uint4*>(src + 8));
     float amax = fmax_nan(amax8(v[0]), amax8(v[1]));
     amax = fmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
@@ -248,8 +248,8 @@ quant_weight_kernel(const __nv_bfloat16* __restrict__ w, uint8_t* __restrict__ q
       if (WIDE) {
         if (has1) load_32b<true>(src + 32 * i * ldw, v[2 * i], v[2 * i + 1]);
       } else {
-        if (has0) v[2 * i] = __ldg(reinterpret_cast<const uint4*>(src + 32 * i * ldw));
-        if (has1) v[2 * i + 1] = __ldg(reinterpret_cast<const uint4*>(src + 32 * i * ldw + 8));
+        if (has0) v[2 * i] = ld_global(reinterpret_cast<const uint4*>(src + 32 * i * ldw));
+        if (has1) v[2 * i + 1] = ld_global(reinterpret_cast<const uint4*>(src + 32 * i * ldw + 8));
       }
     }
   }

@@ -200,3 +200,23 @@ def test_native_module_learns_of_every_status_word(monkeypatch):
     monkeypatch.setattr(torch.Tensor, "is_cuda", True)
     assert runtime.native_for(torch.zeros(1)) is module
     assert told == {7: theirs.data_ptr()}
+
+
+def test_kernels_that_start_early_load_what_others_write_with_ordinary_loads():
+    """A kernel launched with programmatic serialisation begins before the one in front of it has ended, so its operands are
+    not read-only for its lifetime: no __ldg, no ld.global.nc and no const __restrict__ pointer (which the compiler may turn
+    into one) where a file's kernels wait for their predecessor."""
+    import pathlib
+    import re
+
+    waiting = 0
+    for f in sorted((pathlib.Path(pkg.__file__).parent / "csrc").glob("*.cuh")):
+        text = re.sub(r"//[^\n]*", "", f.read_text())
+        if "griddepcontrol.wait" not in text and "pdl_wait" not in text:
+            continue
+        waiting += 1
+        assert "__ldg" not in text and "global.nc" not in text, f.name
+        for body in text.split("__global__")[1:]:
+            if "griddepcontrol.wait" in body or "pdl_wait" in body:
+                assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", body.split("{")[0]), f.name
+    assert waiting >= 2
