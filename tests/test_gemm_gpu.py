@@ -471,3 +471,36 @@ def test_auto_with_a_workspace_that_holds_no_partial_tiles(device, M, N, K):
         assert oracle.max_err_over_rms(out.cpu(), want.cpu()) <= 2e-6
         assert call is rowscale or torch.equal(out, want)      # whole tiles add the K blocks in order, whichever form
         assert call(size - 1) == 6                               # B200FP8_ERR_WORKSPACE
+
+
+def _scales_at(As, offset, ld):
+    """The same scales in a buffer with another base alignment (in floats) and row pitch."""
+    flat = torch.full((offset + As.shape[0] * ld,), float("nan"), device=As.device)
+    view = flat[offset:].view(As.shape[0], ld)[:, :As.shape[1]]
+    view.copy_(As)
+    return view
+
+
+@pytest.mark.parametrize("M,N,K,offset,ld,where", [
+    (1611, 7000, 4208, 0, 33, "copied"),        # 33 scales a row, 2475 tile K blocks of pairs and more: a prep launch copies them
+    (1536, 8192, 4096, 1, 32, "copied"),        # rows of 32, base off by one float
+    (9, 18944, 8320, 0, 65, "copied"),          # up to 16 rows: A is copied too; 128-wide tiles
+    (5, 28672, 11136, 0, 87, "copied"),         # the same on 256-wide ones
+    (300, 384, 2048, 1, 16, "one by one"),      # few enough tiles that a load per K block is the better way
+    (300, 2560, 4096, 2, 32, "one by one"),     # 8-byte aligned: pairs of scales for 128-wide tiles, single ones otherwise
+    (16, 1280, 1664, 3, 13, "one by one")])
+def test_token_scales_wherever_they_are(device, M, N, K, offset, ld, where):
+    """The GEMM kernel reads As in place, in groups where every row is aligned and one by one otherwise, or from a copy that a prep
+    launch makes: the same bits, and those of the fp64 product."""
+    x = torch.randn(M, K, device=device, generator=torch.Generator(device).manual_seed(M + N)).to(torch.bfloat16)
+    w = torch.randn(N, K, device=device, generator=torch.Generator(device).manual_seed(K)).to(torch.bfloat16) * 0.02
+    A, As = pkg.fp8_act_quant(x)
+    B, Bs = pkg.fp8_weight_quant(w)
+    assert (-(-M // 128) * -(-N // 256) * -(-K // 128) > 64 * 148 or N == 18944) == (where == "copied")
+    want = runtime.gemm(A, B, _scales_at(As, 0, -(-As.shape[1] // 4) * 4), Bs, 128, 128, torch.float32)
+    got = runtime.gemm(A, B, _scales_at(As, offset, ld), Bs, 128, 128, torch.float32)
+    runtime.check_device_status()
+    assert torch.equal(got, want)
+    rows = slice(0, M, max(1, M // 200))         # every so many rows keeps the fp64 product small
+    # fp32 accumulation over K blocks, exact fp32 products inside one: a few roundings of 2^-24 each per K block
+    assert _rel(got[rows], A[rows], B, As[rows], Bs) <= 2.0 ** -24 * (2 + -(-K // 128)) ** 0.5 * 4

@@ -115,3 +115,26 @@ def test_rowscale_on_clusters(device, M, N, K):
     assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.float32), out32)
     assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.bfloat16), out32.to(torch.bfloat16))
     runtime.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,form", [(1300, 3584, 2064, 7), (890, 5888, 4592, 7), (1300, 3072, 1040, 6)])
+def test_rowscale_on_cta_pairs_with_odd_row_blocks(device, M, N, K, form):
+    """An odd number of 128-row blocks on 256 x 256 tiles, with whole tiles and with a last wave cut into ranges of 5 and of 9
+    K blocks (shorter and longer than a scale chunk of 8); which form runs is asserted, so that another rule cannot empty this."""
+    import ctypes
+
+    from hf_kernels_helion_b200 import _lib
+
+    ctas = ctypes.c_int(0)
+    assert _lib.load().b200fp8_gemm_auto_form(M, N, K, _lib.CALL_ROWSCALE, ctypes.byref(ctas)) == form and ctas.value == 1
+    A, B, As, Bs = oracle.make_rowscale_inputs(M, N, K, M + N + K)
+    d = [t.to(device) for t in (A, B, As, Bs)]
+    a = (d[0].double() * d[2].double().repeat_interleave(128, 1)[:, :K])
+    ref = a @ (d[1].double() * d[3].double().repeat_interleave(128, 1)[:, :K]).T
+    out32 = runtime.gemm_rowscale(*d, 128, torch.float32)
+    # fp32 accumulation over K blocks, exact fp32 products inside one: a few roundings of 2^-24 each per K block
+    rel = ((out32.double() - ref).norm() / ref.norm()).item()
+    assert rel <= 2.0 ** -24 * (2 + -(-K // 128)) ** 0.5 * 4
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.float32), out32)
+    assert torch.equal(runtime.gemm_rowscale(*d, 128, torch.bfloat16), out32.to(torch.bfloat16))
+    runtime.check_device_status()
