@@ -255,8 +255,8 @@ int make_tmap_u8(CUtensorMap* map, const void* base, int64_t rows, int64_t cols,
 
 // Launch with programmatic stream serialisation: the kernel may be put on the device while the one before it in the
 // stream drains, and waits for it (pdl_wait) before it touches memory. Hides the launch latency between consecutive
-// kernels of a stream: 4096 x 8192 activations 18.4 -> 15.7 us call after call, a row-scaled 512 x 512 x 2048 product (two
-// prep launches) 20.5 -> 17.6. (The weight quantiser, one launch of many blocks, gained nothing.)
+// kernels of a stream: 4096 x 8192 activations 18.4 -> 15.7 us call after call, a row-scaled 512 x 512 x 2048 product, with
+// two prep launches then, 20.5 -> 17.6. (The weight quantiser, one launch of many blocks, gained nothing.)
 template <typename... P, typename... A>
 void launch_pdl(void (*kernel)(P...), dim3 grid, cudaStream_t stream, A... args) {
   cudaLaunchAttribute attr[1];
@@ -398,8 +398,9 @@ TileSkPlan pair_sk_plan(int64_t M, int64_t N, int64_t K, int pairs) {
 // AUTO's estimate of each form's time in us, fitted to graph replays of 46 shapes with 129..8192 rows, 512..28672 columns
 // and 1024..8192 deep (single launches on B200): a start-up, then per wave of tiles the K blocks at the form's rate
 // and the end of a tile (register stores in the split single-CTA form, staged ones otherwise), and 6 us for the
-// fix-up pass of a split last wave. Its choice is 1.5 % slower than the fastest form of each shape in the mean; the rule
-// before it (wave efficiencies, an even number of row blocks for CTA pairs) was 11.5 % slower. For instance, measured
+// fix-up pass of a split last wave. Over 46 other sizes of the same ranges (graph replays, two operand sets) its choice and the
+// cluster form's take 1.0 % more than the fastest of the five in the mean; the worst wrong choice is 209 x 544 x 1408 (128 x
+// 128 tiles 11.1 us, 128 x 256 10.1). For instance, measured
 // 128 x 128 / 128 x 256 / its split tail / pairs / their split tail: 1611 x 7000 x 4208 79.5 / 69.9 / 70.8 / 57.7 / 57.5,
 // 2545 x 1920 x 6272 64.1 / 54.0 / 44.3 / 53.4 / 42.7, 317 x 24832 x 2432 41.9 / 27.6 / 28.2 / 36.5 / 36.5,
 // 1394 x 1536 x 1152 10.7 / 11.1 / 14.8 / 11.1 / 16.0, 4096 x 4096 x 8192 184.3 / 149.3 / 143.2 / 151.6 / 135.0.
@@ -570,8 +571,8 @@ int launch_tile(const void* A, const void* B, GemmArgs args, int64_t lda, int64_
   CUtensorMap ta, tb;
   // Weight-streaming shapes: kernel forms with 16- or 64-row A slots and six or five pipeline stages
   // (measured 3-4 % faster than the 128-row form at N = 28672, K = 8192: 44.5-46 us at M <= 17).
-  // The prep kernel's copy of A has at least 16 rows (M <= 16 goes through a 16-row copy: TMA over the
-  // caller's own 16-row tensor measured 4 % slower than over the copy in the workspace).
+  // A copy of A that the prep kernel makes for M <= 16 has 16 rows. Without a prep launch the box is over the caller's
+  // own rows: a load 4 % slower than from the 16-row copy, and the launch saved is worth more (direct_scales).
   const bool decode = BN == 256 && args.M <= 64 && args.sk_split < 2 && args.n_dst == 1 && !args.mc_store &&
                       args.BsT == nullptr;
   const uint32_t a_rows = !decode ? 128u : args.M <= 16 ? 16u : 64u;

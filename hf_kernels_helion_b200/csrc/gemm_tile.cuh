@@ -1121,7 +1121,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   gemm_tile_body<BN, false, SK>(tmap_a, tmap_b, args, nullptr);
 }
 
-// Cluster split (launch with a cluster dimension of 2, 4 or 8 that divides the grid; one tile per cluster).
+// Cluster split (launch with a cluster dimension of 2 to kClusterMax that divides the grid; one tile per cluster).
 __global__ void __launch_bounds__(TileCfg<128, false>::THREADS, 1)
 gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmArgs args) {

@@ -65,7 +65,7 @@ const at::Tensor* plain_cuda(PyObject* o, at::ScalarType type) {
   const at::Tensor& t = THPVariable_Unpack(o);
   static const uint64_t allowed =
       c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
-                           c10::DispatchKey::AutocastCUDA})   // (the ops have no autocast rule)
+                           c10::DispatchKey::AutocastCUDA})   // (every CUDA tensor has it; autocast that is switched on shows in plain_state)
           .raw_repr();
   if ((t.key_set().raw_repr() & ~allowed) != 0 || !t.is_cuda() || t.scalar_type() != type) return nullptr;
   if (t.requires_grad() && c10::GradMode::is_enabled()) return nullptr;

@@ -163,10 +163,11 @@ int b200fp8_gemm_scatter(const void* A, const void* B, const float* As, const fl
  * reference's second block-FP8 kernel, deep-gemm-helion
  * (deep-gemm-helion/deep-gemm-helion/torch-ext/deep_gemm_helion/fp8.py:13-29:
  * acc += dot(a, b^T) * sA[m, kb][:, None] * sB[n, kb][None, :], bf16 result;
- * torch-ext/deep_gemm_helion/op.py:7-10). Runs on the 128 x 128 tile kernel; the promotion
- * multiplies every accumulator column by its own scale (one multiply more per element than
- * the block-scaled form). Workspace: b200fp8_gemm_rowscale_workspace_bytes(M, N, K) bytes,
- * 256-byte aligned (both scale sets re-laid K-block-major).
+ * torch-ext/deep_gemm_helion/op.py:7-10). Runs on 128 x 128 tiles, on clusters that share
+ * one, or on 256 x 256 tiles of CTA pairs; the promotion multiplies every accumulator column
+ * by its own scale (one multiply more per element than the block-scaled form). Workspace:
+ * b200fp8_gemm_rowscale_workspace_bytes(M, N, K) bytes, 256-byte aligned (both scale sets re-laid
+ * K-block-major, and the partial tiles of a split last wave, without which the same tiles run unsplit).
  */
 int b200fp8_gemm_rowscale(const void* A, const void* B, const float* As, const float* Bs_row, void* C,
                           int64_t M, int64_t N, int64_t K,

@@ -276,16 +276,16 @@ def test_pair_tail_split_k(device, M, N, K):
 
 
 def test_auto_takes_cta_pairs_where_they_pay(device):
-    """AUTO = 256 x 256 tiles on CTA pairs for M > 256 with an even number of 128-row blocks, when the
-    destination takes 16-byte rows (the output is then staged and stored by TMA); otherwise the
-    single-CTA choice. Either way the bits are those of the single-CTA kernel."""
+    """AUTO takes 256 x 256 tiles on CTA pairs where their estimated time is the smallest, when the destination takes
+    16-byte rows (the output is then staged and stored by TMA). Whole tiles have the bits of the single-CTA
+    kernel, whichever they are; forms that cut K (split tails, clusters) add in another order."""
     lib = _lib.load()
     pair = _lib.VARIANT_NAMES["pair256_split"]
     assert lib.b200fp8_gemm_pair_clusters() > 0
     assert lib.b200fp8_gemm_pick_variant(8192, 18432, 7168) == _lib.VARIANT_NAMES["pair256_split_sk"]   # 10 tiles in the 32nd wave
     assert lib.b200fp8_gemm_pick_variant(2048, 2048, 4096) == pair                                     # 64 tiles: one wave, nothing to split
     assert lib.b200fp8_gemm_pick_variant(4096, 4096, 8192) == _lib.VARIANT_NAMES["pair256_split_sk"]   # 34 tiles in the last wave of 74
-    assert lib.b200fp8_gemm_pick_variant(640, 4096, 1024) != pair      # five row blocks
+    assert lib.b200fp8_gemm_pick_variant(640, 4096, 1024) != pair      # 80 tiles of 128 x 256 are one wave of SMs, 48 pair tiles leave a third idle
     assert lib.b200fp8_gemm_pick_variant(256, 28672, 8192) == pair
     assert lib.b200fp8_gemm_pick_variant(128, 28672, 8192) == _lib.VARIANT_TILE256
     assert lib.b200fp8_gemm_pick_variant(200, 128, 512) == _lib.VARIANT_NAMES["tile128"]
@@ -367,8 +367,8 @@ def _rel(out, A, B, As, Bs):
                                    (1024, 1024, 8192), (1611, 2000, 1168), (2545, 1920, 6272)])
 def test_auto_on_small_and_ragged_products(device, M, N, K):
     """Products whose tiles leave SMs idle run as clusters that share a tile (ranges of two K blocks and more, uneven ones, a
-    short last K block, rows and columns that fill no tile, rows of the result that are not 16-byte multiples); odd
-    numbers of row blocks run on CTA pairs. Into a view with sentinels around it, twice the same bits."""
+    short last K block, rows and columns that fill no tile, rows of the result that are not 16-byte multiples); the largest
+    leave little idle and run on other forms. Into a view with sentinels around it, twice the same bits."""
     A, B, As, Bs = _dev(oracle.make_quantised_inputs(M, N, K, M + N), device)
     buf = torch.full((M + 2, N + 24), 7.0, dtype=torch.float32, device=device)
     out32 = runtime.gemm(A, B, As, Bs, 128, 128, torch.float32, out=buf[1:M + 1, 8:8 + N])

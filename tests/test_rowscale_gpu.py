@@ -84,9 +84,9 @@ def test_legacy_call_form_of_the_reference_harness(device):
 @pytest.mark.parametrize("M,N,K", [(256, 256, 128), (257, 1100, 1152), (512, 4104, 1040), (1000, 9472, 2064), (2100, 2304, 640),
                                    (256, 4096, 4096), (1000, 3008, 4112)])
 def test_rowscale_on_cta_pairs(device, M, N, K):
-    """Sizes at which the 256 x 256 form runs or borders on: odd numbers of 128-row blocks, columns and K blocks that fill no
-    tile and no scale chunk (8 K blocks), rows that are not 16-byte multiples (register stores, 128 x 128 tiles), whole
-    waves, a last wave split along K whose ranges start inside a chunk, chunks recycled over several tiles."""
+    """Sizes at which the 256 x 256 form runs or borders on: columns and K blocks that fill no tile and no scale chunk (8 K
+    blocks), rows that are not 16-byte multiples (register stores, 128 x 128 tiles), whole waves, chunks recycled over
+    several tiles. (Odd row blocks and split tails: test_rowscale_on_cta_pairs_with_odd_row_blocks.)"""
     A, B, As, Bs = oracle.make_rowscale_inputs(M, N, K, M + N + K)
     d = [t.to(device) for t in (A, B, As, Bs)]
     a = (d[0].double() * d[2].double().repeat_interleave(128, 1)[:, :K])
